@@ -309,9 +309,9 @@ extern "C" int fb_builder_create(int device, fb_builder** out) {
   for (int mode = 0; mode < 2; ++mode)
     for (int pass = 0; pass < 4; ++pass)
       for (int tpt : {1, 2})
-        for (int variant = 0; variant < 12; ++variant) {
-        // variants 0..5 (density: occupancy + clamped tables), of order 2 or not
-        const void* k = fb::kernel_for(mode == 1, pass, tpt, variant % 6, variant >= 6);
+        for (int variant = 0; variant < 2 * fb::kDensVariants; ++variant) {
+        // every variant (density: occupancy, clamped tables, arcs), of order 2 or not
+        const void* k = fb::kernel_for(mode == 1, pass, tpt, variant % fb::kDensVariants, variant >= fb::kDensVariants);
         cudaFuncAttributes kfa;
         if (cudaFuncGetAttributes(&kfa, k) != cudaSuccess ||
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -492,6 +492,7 @@ struct PlannedLaunch {
   int tpt;
   int variant;
   int order;
+  int arc_rows;
   int nseg;
   int seg_njobs[fb::kMaxSegments];
   int seg_total[fb::kMaxSegments];
@@ -594,14 +595,41 @@ void plan_group(Plan& P, const std::vector<DevAtmo>& A, const std::vector<int>& 
     std::vector<int> jobs;
     for (int j : group)
       if (A[j].order >= n) jobs.push_back(j);
+    // orders >= 3: the atmospheres that go by arcs have a launch of their own
+    // (each atmosphere's kernel depends on its own sizes alone)
+    std::vector<int> arcs, direct;
+    for (int j : jobs) (n >= 3 && A[j].arcs ? arcs : direct).push_back(j);
+    if (!arcs.empty()) {
+      PlannedLaunch D = mk(fb::kPassDensity, n);
+      std::vector<int> t0, t1;
+      int gi = 0;
+      for (int j : arcs) {
+        const DevAtmo& a = A[j];
+        const fb::ArcShape sh = fb::arc_shape(a.sc_r, a.sc_mu, a.sc_mus, a.sc_nu);
+        gi = std::max(gi, sh.gi);
+        t0.push_back(sh.tiles);
+        t1.push_back(fb::tiles_indirect(a.ir_mus, a.ir_r, a.irr_n, a.sc_nu, a.W, false));
+        D.texels += (uint64_t)a.W * a.sc_mu * a.sc_r + (uint64_t)a.ir_mus * a.ir_r;
+      }
+      D.block = fb::kArcThreads;
+      D.variant = fb::arc_variant(gi);
+      D.arc_rows = fb::arc_launch_rows(arcs, [&](int j) -> const DevAtmo& { return A[j]; }, fb::arc_ctas(gi), &D.smem);
+      for (int j : arcs)
+        D.smem = std::max(D.smem, fb::indirect_smem(A[j].irr_n, A[j].sc_nu, A[j].W, A[j].ir_mus, false));
+      add_segment(P, D, 0, arcs, t0);
+      add_segment(P, D, 1, arcs, t1);
+      D.nseg = 2;
+      P.launches.push_back(D);
+    }
+    if (!direct.empty()) {
     PlannedLaunch D = mk(fb::kPassDensity, n);
     std::vector<int> t0, t1;
     // the tuned variant (occupancy, + kDensClamped for exact-size tables); the
     // exact-size tables also wherever the power-of-two ones do not fit
-    const int tuned = launch_variant(A, jobs, tun, mixed, true);
+    const int tuned = launch_variant(A, direct, tun, mixed, true);
     bool cl = tuned >= fb::kDensClamped;
-    for (int j : jobs) cl |= fb::density_smem(A[j], n == 2, mixed, false) > smem_limit;
-    for (int j : jobs) {
+    for (int j : direct) cl |= fb::density_smem(A[j], n == 2, mixed, false) > smem_limit;
+    for (int j : direct) {
       const DevAtmo& a = A[j];
       t0.push_back(fb::tiles_density(a));
       t1.push_back(fb::tiles_indirect(a.ir_mus, a.ir_r, a.irr_n, a.sc_nu, a.W, n - 1 == 1));
@@ -609,11 +637,12 @@ void plan_group(Plan& P, const std::vector<DevAtmo>& A, const std::vector<int>& 
       D.smem = std::max(D.smem, fb::indirect_smem(a.irr_n, a.sc_nu, a.W, a.ir_mus, n - 1 == 1));
       D.texels += (uint64_t)a.W * a.sc_mu * a.sc_r + (uint64_t)a.ir_mus * a.ir_r;
     }
-    add_segment(P, D, 0, jobs, t0);
-    add_segment(P, D, 1, jobs, t1);
+    add_segment(P, D, 0, direct, t0);
+    add_segment(P, D, 1, direct, t1);
     D.nseg = 2;
     D.variant = tuned % fb::kDensClamped + (cl ? fb::kDensClamped : 0);
     P.launches.push_back(D);
+    }
     PlannedLaunch M = mk(fb::kPassMultiple, n);
     std::vector<int> tm;
     for (int j : jobs) M.block = std::max(M.block, fb::ms_threads(A[j].W));
@@ -688,6 +717,8 @@ void fill_devatmo(DevAtmo& d, const fb_params& p, const fbi::Tuning& tun) {
   const fbi::TuneEntry* te = fbi::tuning_find(tun, d.sc_r, d.sc_mu, d.sc_mus, d.sc_nu, (int)p.precision);
   d.dens_S = te ? te->dens_S : 0;
   d.dens_chunk = te ? te->dens_chunk : 0;
+  d.arc_ke = fb::arc_ground_knots(d.ir_mus, d.bottom, d.Hd);
+  d.arcs = fb::arc_use(d);
 }
 
 }  // namespace
@@ -813,6 +844,7 @@ int build(fb_builder* b, cudaStream_t s, const fb_params* params, uint32_t count
     R.args.atm = d_atm;
     R.args.nseg = L.nseg;
     R.args.order = L.order;
+    R.args.arc_rows = L.arc_rows;
     R.args.counter = d_cnt + li;
     int total = 0;
     for (int sidx = 0; sidx < L.nseg; ++sidx) {

@@ -1,0 +1,548 @@
+// fb_density_arcs.cuh — scattering density of orders >= 3 by arcs (included by
+// fb_passes.cuh).
+//
+// On a theta row of the sphere grid the incident radiance is a piecewise
+// linear function f of the position t = (nu_size - 1) / 2 (nu_i + 1) of the
+// direction's sun angle in the previous order's table, whose knots are the
+// table's nu texels; for rows that meet the ground, the bounce is piecewise
+// linear in t as well (fb_passes.cuh, dens_row), with the irradiance texels as
+// knots. With omega_s at azimuth phi_s, t = base + s cos(phi - phi_s), so that
+// a knot t_k cuts the row's azimuths into an arc of half width alpha_k =
+// acos((t_k - base) / s) around phi_s and the rest, and
+//   sum_m c_m f(t_m) = sum_m c_m line(t_m)
+//                      + sum_k dB_k sum_{m in arc k} c_m (t_m - t_k),
+// with the phase weights c_m of the row's directions, the line of the lowest
+// interval and the slope changes dB_k. The inner sums follow from running
+// sums over m of c_m, c_m cos phi_m and c_m sin phi_m at the two ends of the
+// arc. This is the sum over all directions, regrouped: a row costs as many
+// steps as it has knots (4-5 on average for 8 nu slices) instead of 32
+// directions. Measured against the direct sums (tile_density), density of order
+// 3: 16 default atmospheres 6.46 -> 2.25 ms, one of twice the size in every
+// dimension (16 nu slices) 6.58 -> 4.1 ms, one default atmosphere 0.461 -> 0.175
+// ms, with the same errors against FP64. Bound by the shared-memory pipe (76 %
+// of its wavefronts; six 8-byte loads per texel and knot) and, between the
+// batches of theta rows, by the latency of building the next ones.
+//
+// The weights are c_m = A t1_m + B t1_m rs3_m per channel (PhaseCoef) with A
+// and B constant in the tile: the running sums are kept for t1 and t1 rs3 and
+// every texel sums its six products, combined once at the end.
+//
+// Tile: one r slice, 32 mu rows (a lane each: the running sums belong to the
+// lane's mu and lie in its own shared-memory banks, so no lookup conflicts) and
+// S mu_s columns (a warp for up to kArcMaxGroup of a column's nu texels: the
+// row's knots are the same for the whole warp, read as broadcasts). The texels
+// at nu = -1 and 1, and every texel whose nu the clamp of scattering.h:134-136
+// moves, have omega_s in the plane of omega (phi_s = 0 or pi): those arcs are
+// symmetric and take one lookup of four sums, and one evaluation per column
+// serves all of a lane's clamped texels.
+#pragma once
+
+namespace fb {
+
+constexpr int kArcWarps = 8, kArcThreads = 32 * kArcWarps;
+constexpr int kArcMaxGroup = 7;    // nu texels per thread besides the two ends
+constexpr int kArcMaxRows = 4;     // theta rows whose running sums are held at a time
+constexpr int kArcStage = 36;      // stride of a staged column of 32 results (36: rows of 8 columns x 4 rows on distinct banks)
+constexpr int kArcMaxIrMus = 512;  // the ground irradiance row is held in shared memory
+
+struct ArcShape {
+  int NG, gi;  // warps per column, nu texels (ends aside) per warp
+  int S;       // mu_s columns per tile
+  int scols, ychunks, tiles;
+};
+__host__ __device__ inline ArcShape arc_shape(int sc_r, int sc_mu, int sc_mus, int sc_nu) {
+  ArcShape d;
+  const int inner = sc_nu - 2;
+  d.NG = max(1, (inner + kArcMaxGroup - 1) / kArcMaxGroup);
+  d.gi = (inner + d.NG - 1) / d.NG;
+  d.S = max(1, min(sc_mus, kArcWarps / d.NG));
+  d.scols = (sc_mus + d.S - 1) / d.S;
+  d.ychunks = (sc_mu + 31) / 32;
+  d.tiles = sc_r * d.scols * d.ychunks;
+  return d;
+}
+
+// Knots of the ground irradiance within one theta row, at most: the row spans
+// (ir_mus - 1) (dg / R) sin t sin s texels, dg <= H.
+inline int arc_ground_knots(int ir_mus, double bottom, double H) {
+  const double span = (ir_mus - 1) * (H / bottom);
+  return span < ir_mus ? (int)span + 2 : ir_mus;
+}
+__host__ __device__ inline int arc_knots(int sc_nu, int ke) { return max(1, sc_nu - 2 + ke); }
+
+struct ArcLayout {
+  float2* T;       // LB x (2 NT + 1) x 3 x 32 lanes: running sums (c, c x) of t1, of t1 rs3, (c y of both)
+  float* stage;    // the tile's results, in the place of T: 3 x nu x S x kArcStage
+  float4* V;       // S x NT x nu: the previous order's table at the rows' entries
+  float4* ka;      // S x LB x KC: knots: alpha (in directions), base - t_k, dB.x, dB.y
+  float* kb;       // S x LB x KC: dB.z
+  float4* f0;      // S x LB x 2: the lowest line's value at base, the number of knots; its slope
+  float4* E;       // ir_mus: ground irradiance row
+  float2* dir;     // NT: cos phi, sin phi
+  float2* ts;      // NT: hP sin t, ground table position per t: A
+  DensTheta* th;   // NT
+  Axis* tay;       // NT
+  Axis* kax;       // S x nu
+  float4* col;     // S: mu_s, sin s, 1 - mu_s^2 and its low part
+  float* col2;     // S: the low part of mu_s
+  float2* nu;      // nu: MIXED: the texels' nu as a sum of two floats
+};
+__host__ __device__ inline size_t arc_layout(unsigned char* base, int NT, int nu, int ir_mus, int S, int KC, int LB,
+                                             ArcLayout* L) {
+  size_t o = 0;
+  auto take = [&](size_t bytes) {
+    size_t at = o;
+    o = align16(o + bytes);
+    return at;
+  };
+  const size_t t_bytes = sizeof(float2) * LB * (2 * NT + 1) * 3 * 32, st_bytes = sizeof(float) * 3 * nu * S * kArcStage;
+  const size_t o_T = take(t_bytes > st_bytes ? t_bytes : st_bytes);
+  const size_t o_V = take(sizeof(float4) * S * NT * nu), o_ka = take(sizeof(float4) * S * LB * KC);
+  const size_t o_kb = take(sizeof(float) * S * LB * KC), o_f0 = take(sizeof(float4) * S * LB * 2);
+  const size_t o_E = take(sizeof(float4) * ir_mus), o_dir = take(sizeof(float2) * NT), o_ts = take(sizeof(float2) * NT);
+  const size_t o_th = take(sizeof(DensTheta) * NT), o_tay = take(sizeof(Axis) * NT);
+  const size_t o_kax = take(sizeof(Axis) * S * nu), o_col = take(sizeof(float4) * S);
+  const size_t o_col2 = take(sizeof(float) * S), o_nu = take(sizeof(float2) * nu);
+  if (L) {
+    L->T = (float2*)(base + o_T);
+    L->stage = (float*)(base + o_T);
+    L->V = (float4*)(base + o_V);
+    L->ka = (float4*)(base + o_ka);
+    L->kb = (float*)(base + o_kb);
+    L->f0 = (float4*)(base + o_f0);
+    L->E = (float4*)(base + o_E);
+    L->dir = (float2*)(base + o_dir);
+    L->ts = (float2*)(base + o_ts);
+    L->th = (DensTheta*)(base + o_th);
+    L->tay = (Axis*)(base + o_tay);
+    L->kax = (Axis*)(base + o_kax);
+    L->col = (float4*)(base + o_col);
+    L->col2 = (float*)(base + o_col2);
+    L->nu = (float2*)(base + o_nu);
+  }
+  return o;
+}
+__host__ __device__ inline size_t arc_smem(const DevAtmo& a, int LB) {
+  const ArcShape s = arc_shape(a.sc_r, a.sc_mu, a.sc_mus, a.sc_nu);
+  return arc_layout(nullptr, a.dens_n, a.sc_nu, a.ir_mus, s.S, arc_knots(a.sc_nu, a.arc_ke), LB, nullptr);
+}
+
+// CTAs per SM that the kernel of `gi` nu texels per thread is compiled for, and
+// the shared memory each may then use (a block reserves 1 KB beside its own).
+__host__ __device__ constexpr int arc_ctas(int gi) { return gi <= 2 ? 3 : 2; }
+constexpr size_t arc_smem_per_cta(int ctas) { return 228 * 1024 / ctas - 1024 - 64; }
+
+// Whether an atmosphere's orders >= 3 go by arcs: where a row has fewer knots
+// than half its directions (a knot costs as much as one and a half to two
+// directions) and the tables of one theta row fit beside another CTA.
+inline bool arc_use(const DevAtmo& a) {
+  if (a.ir_mus > kArcMaxIrMus) return false;
+  // knots of a row on average: the sines shorten its range of nu, and only the
+  // rows next to the horizon see much of the ground row
+  const int knots = (6 * (a.sc_nu - 2)) / 10 + a.arc_ke / 6;
+  return knots <= a.dens_n && arc_smem(a, 1) <= arc_smem_per_cta(2);
+}
+// Theta rows per batch of a launch over `jobs` (the largest that fits) and the
+// launch's shared memory for them.
+template <class Jobs, class Get>
+inline int arc_launch_rows(const Jobs& jobs, Get get, int ctas, size_t* smem) {
+  for (int LB = kArcMaxRows;; --LB) {
+    *smem = 0;
+    for (const auto& j : jobs) *smem = arc_smem(get(j), LB) > *smem ? arc_smem(get(j), LB) : *smem;
+    if (LB == 1 || *smem <= arc_smem_per_cta(ctas)) return LB;
+  }
+}
+
+// e / d for 0 <= e < 2^16, given 1 / d (an integer division costs some twenty
+// instructions); the half keeps the quotient off the integers.
+__device__ __forceinline__ int arc_div(int e, float inv_d) { return (int)((float(e) + 0.5f) * inv_d); }
+
+// One running-sum entry: field 0 (c, c x) of t1, 1 of t1 rs3, 2 (c y) of both.
+template <int FIELD> __device__ __forceinline__ float2 arc_ld(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2 + %3];" : "=f"(v.x), "=f"(v.y) : "r"(addr), "n"(FIELD * 256));
+  return v;
+}
+constexpr uint32_t kArcEntryBytes = 3 * 32 * sizeof(float2);
+// Byte offset of the entry at position x >= 0: the number of directions of a
+// half circle (phi_m = (m + 1/2) pi / NT) below the angle x pi / NT is x
+// rounded to an integer, taken through the float adder (line_pos). base: the
+// table's address less kRoundMagicBits entries.
+__device__ __forceinline__ uint32_t arc_entry(float x, uint32_t base) {
+  return (uint32_t)__float_as_int(x + kRoundMagic) * kArcEntryBytes + base;
+}
+
+template <bool MX, int GI>
+__device__ void tile_density_arcs(const DevAtmo& a, int order, int tile, int LB, unsigned char* smem) {
+  const int NT = a.dens_n, n = a.sc_nu;
+  const ArcShape sh = arc_shape(a.sc_r, a.sc_mu, a.sc_mus, n);
+  const int KE = a.arc_ke, KC = arc_knots(n, KE), NE = 2 * NT + 1;
+  const int zi = tile / (sh.scols * sh.ychunks);
+  const int rem = tile % (sh.scols * sh.ychunks);
+  const int s0 = (rem / sh.ychunks) * sh.S, y0 = (rem % sh.ychunks) * 32;
+  const int ns = min(sh.S, a.sc_mus - s0), ny = min(32, a.sc_mu - y0);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  ArcLayout L;
+  arc_layout(smem, NT, n, a.ir_mus, sh.S, KC, LB, &L);
+  const float hP = 0.5f * float(n - 1), hE = 0.5f * float(a.ir_mus - 1);
+  const DensZ zr = a.g_z[zi];
+  const float r = zr.r;
+  const Axis s_az = bounded_axis(zr.az, a.sc_r), s_irx = bounded_axis(zr.irx, a.ir_r);
+  // --- the tile's rows and columns from the geometry tables, the ground irradiance row
+  for (int k = tid; k < NT + ns * n + a.ir_mus; k += kArcThreads) {
+    if (k < NT) {
+      const ThetaRec t = a.g_th[(size_t)zi * NT + k];
+      L.th[k] = t.th;
+      L.tay[k] = bounded_axis(t.tay, a.sc_mu);
+      const float phi = (float(k) + 0.5f) * (kPiF / float(NT));
+      L.dir[k] = make_float2(cosf(phi), sinf(phi));
+      L.ts[k] = make_float2(hP * sinf((float(k) + 0.5f) * (kPiF / float(NT))), hE * (t.th.dg / a.bottom) / hP);
+    } else if (k < NT + ns * n) {
+      const int c = (k - NT) / n, j = (k - NT) - c * n;
+      const ColGeo& cg = a.g_cols[s0 + c];
+      if (j == 0) {
+        L.col[c] = make_float4(cg.mu_s, sqrtf(gmax(cg.one_m_mus2, 0.0f)), cg.one_m_mus2,
+                               MX ? (float)(cg.one_m_mus2d - (double)cg.one_m_mus2) : 0.f);
+        L.col2[c] = MX ? (float)(cg.mu_sd - (double)cg.mu_s) : 0.f;
+      }
+      if (MX && c == 0) {
+        const ColGeo& cn = a.g_cols[j * a.sc_mus];
+        L.nu[j] = make_float2(cn.nu_raw, (float)(cn.nu_rawd - (double)cn.nu_raw));
+      }
+      L.kax[k - NT] = MX ? axis_texel(double(j) * a.sc_mus + cg.t_musd, a.W)
+                         : make_axis((float(j) + cg.u_mus) / float(n), a.W);
+    } else {
+      const int e = k - NT - ns * n;
+      const float4* E = a.dirr[order & 1];  // irradiance of order n - 2
+      const float4 e0 = E[s_irx.i0 * a.ir_mus + e], e1 = E[s_irx.i1 * a.ir_mus + e];
+      const float fy = s_irx.f;
+      L.E[e] = make_float4(fmaf(e1.x - e0.x, fy, e0.x), fmaf(e1.y - e0.y, fy, e0.y), fmaf(e1.z - e0.z, fy, e0.z), 0.f);
+    }
+  }
+  // --- the lane's mu and this warp's texels: azimuth of omega_s in units of
+  // the direction spacing, omega_s' components (scattering_density.comp:28-32)
+  const int c = warp / sh.NG, grp = warp - c * sh.NG;
+  const bool has_col = c < ns;
+  const bool has_lo = grp == 0, has_hi = grp == sh.NG - 1;
+  const int y = y0 + min(lane, ny - 1), row = zi * a.sc_mu + y;
+  const int k0 = 1 + grp * sh.gi, kn = has_col ? min(sh.gi, n - 1 - k0) : 0;  // nu texels k0 .. k0 + kn - 1
+  const RowGeo& rg = a.g_rows[row];
+  const float mu = rg.mu, ox = MX ? sqrtf(rg.om_hi) : sqrtf(1.0f - mu * mu);
+  const float mu_lo = rg.mu_lo, om_hi = rg.om_hi, om_lo = rg.om_lo;
+  __syncthreads();
+  float phi[GI], sx[GI], sy[GI];
+  int cls = 0;  // two bits per texel: 1 clamped low, 2 clamped high
+  {
+    const float4 cf = L.col[has_col ? c : 0];
+    const float mu_s = cf.x, ss = cf.y;
+    // MIXED: delta = nu - mu mu_s and sun_y^2 = (sin^2 sin_s^2 - delta^2) /
+    // sin^2 cancel where omega_s is near omega's plane; in sums of two floats
+    // they keep 1e-13 of their terms, as in FP64 (which this part runs at a
+    // 64th of the rate)
+    float ph = 0.f, pl = 0.f, mh = 0.f, ml = 0.f, isom = 0.f;
+    if (MX) {
+      const float p2 = cf.z, p2l = cf.w, ms_lo = L.col2[has_col ? c : 0];
+      ph = om_hi * p2;
+      pl = fmaf(om_hi, p2, -ph) + (om_hi * p2l + om_lo * p2);
+      mh = mu * mu_s;
+      ml = fmaf(mu, mu_s, -mh) + (mu * ms_lo + mu_lo * mu_s);
+      isom = om_hi > 0.0f ? rsqrtf(om_hi) : 0.0f;
+    } else {
+      const float sq32 = sqrtf((1.0f - mu * mu) * cf.z);
+      ph = mu * mu_s - sq32;  // the range of nu
+      mh = mu * mu_s + sq32;
+    }
+#pragma unroll
+    for (int j = 0; j < GI; ++j) {
+      phi[j] = sx[j] = sy[j] = 0.f;
+      if (j < kn) {
+        bool lo, hi;
+        if (MX) {
+          const float2 nu = L.nu[k0 + j];
+          const float dh = nu.x - mh, t = dh - nu.x;
+          const float dl = ((nu.x - (dh - t)) - (mh + t)) + (nu.y - ml);
+          const float qh = dh * dh, ql = fmaf(dh, dh, -qh) + 2.0f * dh * dl;
+          const float rest = (ph - qh) + (pl - ql);
+          lo = rest < 0.0f && dh < 0.0f;
+          hi = rest < 0.0f && dh >= 0.0f;
+          sx[j] = (dh + dl) * isom;
+          sy[j] = om_hi > 0.0f ? sqrtf(fmaxf(rest, 0.0f)) * isom : ss;
+        } else {
+          const float nu = a.g_cols[(k0 + j) * a.sc_mus + s0 + c].nu_raw;
+          lo = nu < ph;
+          hi = nu > mh;
+          sx[j] = ox == 0.0f ? 0.0f : (nu - mu * mu_s) / ox;
+          sy[j] = sqrtf(gmax(1.0f - sx[j] * sx[j] - mu_s * mu_s, 0.0f));
+        }
+        cls |= (lo ? 1 : hi ? 2 : 0) << (2 * j);
+        // clamped so that a NaN cannot leave the running sums' table
+        phi[j] = fminf(fmaxf(atan2f(sy[j], sx[j]) * (float(NT) / kPiF), 0.0f), float(NT));
+      }
+    }
+  }
+  // the previous order's table at the tile's r, columns and theta rows
+  {
+    // columns fastest: neighbouring columns are neighbouring texels
+    const float inv_n = 1.0f / float(n), inv_ns = 1.0f / float(ns);
+    for (int e = tid; e < ns * NT * n; e += kArcThreads) {
+      const int q = arc_div(e, inv_ns), cc = e - q * ns, l = arc_div(q, inv_n), k = q - l * n;
+      const float3 v = fetch3(a.dms, a.W, a.sc_mu, L.kax[cc * n + k], L.tay[l], s_az);
+      L.V[(cc * NT + l) * n + k] = make_float4(v.x, v.y, v.z, 0.f);
+    }
+  }
+  float3 acc1[GI], acc2[GI], lo1, lo2, hi1, hi2, com1, com2;
+#pragma unroll
+  for (int j = 0; j < GI; ++j) acc1[j] = acc2[j] = make_float3(0.f, 0.f, 0.f);
+  lo1 = lo2 = hi1 = hi2 = com1 = com2 = make_float3(0.f, 0.f, 0.f);
+  const float g = a.g, g1 = 1.0f + g * g, g2 = 2.0f * g;
+  __syncthreads();
+  uint32_t Tlane = (uint32_t)__cvta_generic_to_shared(L.T) + lane * (uint32_t)sizeof(float2);
+  asm volatile("" : "+r"(Tlane));  // held in a register rather than formed again at each use
+  for (int l0 = 0; l0 < NT; l0 += LB) {
+    const int nl = min(LB, NT - l0);
+    const float inv_nl = 1.0f / float(nl);
+    if (warp < LB) {
+      // running sums of row l0 + warp: entry e holds the sums over the
+      // directions below the angle e pi / NT; past the half circle they follow
+      // from symmetry (c and cos even, sin odd in phi)
+      if (warp < nl) {
+        const int l = l0 + warp;
+        const DensTheta t = L.th[l];
+        const float st = L.ts[l].x, mu_ct = mu * t.cos_t, oxs = ox / hP;
+        float2* Tw = L.T + (size_t)warp * NE * 96 + lane;
+        float2 s1 = make_float2(0.f, 0.f), s2 = s1, s3 = s1;
+        Tw[0] = Tw[32] = Tw[64] = s1;
+#pragma unroll 4
+        for (int m = 0; m < NT; ++m) {
+          const float2 d = L.dir[m];
+          const float dx = d.x * st, dy = d.y * st;
+          const float nu2 = fmaf(oxs, dx, mu_ct);
+          const float c1 = fmaf(nu2, nu2, 1.0f) * t.domega;
+          const float rs = rsqrt_pos(fmaf(-g2, nu2, g1));
+          const float c2 = c1 * (rs * rs * rs);
+          s1.x += c1;
+          s1.y = fmaf(c1, dx, s1.y);
+          s2.x += c2;
+          s2.y = fmaf(c2, dx, s2.y);
+          s3.x = fmaf(c1, dy, s3.x);
+          s3.y = fmaf(c2, dy, s3.y);
+          float2* e = Tw + (m + 1) * 96;
+          e[0] = s1;
+          e[32] = s2;
+          e[64] = s3;
+        }
+#pragma unroll 4
+        for (int m = 0; m < NT; ++m) {
+          const float2* e = Tw + m * 96;
+          float2* o = Tw + (2 * NT - m) * 96;
+          const float2 v1 = e[0], v2 = e[32];
+          o[0] = make_float2(2.0f * s1.x - v1.x, 2.0f * s1.y - v1.y);
+          o[32] = make_float2(2.0f * s2.x - v2.x, 2.0f * s2.y - v2.y);
+          o[64] = e[64];
+        }
+      }
+    } else {
+      const int tk = tid - 32 * LB, nk = kArcThreads - 32 * LB;
+      // eight lanes per (column, theta row) take its knots in turn
+      for (int pr = tk >> 3; pr < ns * nl; pr += nk >> 3) {
+        const int cc = arc_div(pr, inv_nl), l = pr - cc * nl;
+        const DensTheta t = L.th[l0 + l];
+        const float4 cs = L.col[cc];
+        const float2 ts = L.ts[l0 + l];
+        const float base = hP * fmaf(t.cos_t, cs.x, 1.0f), s = ts.x * cs.y;
+        const float4* V = L.V + (cc * NT + l0 + l) * n;
+        // the intervals of the lowest and the highest position of the row
+        const float tlo = base - s, thi = base + s;
+        const int klo = min(max((int)floorf(tlo), 0), n - 2), khi = min(max((int)floorf(thi), klo), n - 2);
+        const int np = khi - klo;
+        // ground: position A t + B in the irradiance row
+        const float A = ts.y;
+        const float B = hE * (1.0f - t.dg / a.bottom + (r / a.bottom) * cs.x);
+        const int em = a.ir_mus - 2;
+        const int elo = min(max((int)floorf(fmaf(A, tlo, B)), 0), em), ehi = min(max((int)floorf(fmaf(A, thi, B)), elo), em);
+        const int ne = t.ground ? min(ehi - elo, KE) : 0;
+        for (int slot = tk & 7; slot < np + ne; slot += 8) {
+          const int o = (cc * LB + l) * KC + slot;
+          float tk_;
+          float3 d;
+          if (slot < np) {
+            const int k = klo + 1 + slot;
+            const float4 v0 = V[k - 1], v1 = V[k], v2 = V[k + 1];
+            tk_ = float(k);
+            d = make_float3((v2.x - v1.x) - (v1.x - v0.x), (v2.y - v1.y) - (v1.y - v0.y), (v2.z - v1.z) - (v1.z - v0.z));
+          } else {
+            const int k = elo + 1 + slot - np;
+            const float4 v0 = L.E[k - 1], v1 = L.E[k], v2 = L.E[k + 1];
+            tk_ = (float(k) - B) / A;
+            d = make_float3(t.tgx * A * ((v2.x - v1.x) - (v1.x - v0.x)), t.tgy * A * ((v2.y - v1.y) - (v1.y - v0.y)),
+                            t.tgz * A * ((v2.z - v1.z) - (v1.z - v0.z)));
+          }
+          const float co = fminf(fmaxf((tk_ - base) / s, -1.0f), 1.0f);
+          const float al = fminf(fmaxf(acosf(co) * (float(NT) / kPiF), 0.0f), float(NT));
+          L.ka[o] = make_float4(al, base - tk_, d.x, d.y);
+          L.kb[o] = d.z;
+        }
+        if ((tk & 7) == 0) {
+          const float4 v0 = V[klo], v1 = V[klo + 1];
+          float3 b = make_float3(v1.x - v0.x, v1.y - v0.y, v1.z - v0.z);
+          const float f = base - float(klo);
+          float3 v = make_float3(fmaf(f, b.x, v0.x), fmaf(f, b.y, v0.y), fmaf(f, b.z, v0.z));
+          if (t.ground) {
+            const float4 e0 = L.E[elo], e1 = L.E[elo + 1];
+            const float fe = fmaf(A, base, B) - float(elo);
+            const float3 be = make_float3(e1.x - e0.x, e1.y - e0.y, e1.z - e0.z);
+            v.x = fmaf(t.tgx, fmaf(fe, be.x, e0.x), v.x);
+            v.y = fmaf(t.tgy, fmaf(fe, be.y, e0.y), v.y);
+            v.z = fmaf(t.tgz, fmaf(fe, be.z, e0.z), v.z);
+            b.x = fmaf(t.tgx * A, be.x, b.x);
+            b.y = fmaf(t.tgy * A, be.y, b.y);
+            b.z = fmaf(t.tgz * A, be.z, b.z);
+          }
+          const int p = 2 * (cc * LB + l);
+          L.f0[p] = make_float4(v.x, v.y, v.z, __int_as_float(np + ne));
+          L.f0[p + 1] = make_float4(b.x, b.y, b.z, 0.f);
+        }
+      }
+    }
+    __syncthreads();
+    if (has_col) {
+      const float ssn = L.col[c].y;
+      for (int l = 0; l < nl; ++l) {
+        const int pr = c * LB + l;
+        const float4 f0 = L.f0[2 * pr], b0 = L.f0[2 * pr + 1];
+        const int cnt = __float_as_int(f0.w);
+        uint32_t Tr = Tlane + (uint32_t)(l * NE) * kArcEntryBytes;
+        const uint32_t Ttot = Tr + (uint32_t)(2 * NT) * kArcEntryBytes;
+        Tr -= (uint32_t)kRoundMagicBits * kArcEntryBytes;
+        // through a shuffle, so that the assembler sees a value and not a sum:
+        // it would add the terms anew for each of the loads below
+        Tr = __shfl_sync(0xffffffffu, Tr, lane);
+        const float2 w1 = arc_ld<0>(Ttot), w2 = arc_ld<1>(Ttot);  // the whole row
+        com1 = fma3(make_float3(f0.x, f0.y, f0.z), make_float3(w1.x, w1.x, w1.x), com1);
+        com2 = fma3(make_float3(f0.x, f0.y, f0.z), make_float3(w2.x, w2.x, w2.x), com2);
+        auto slope = [&](float x, float3& s1, float3& s2) {
+          const float x1 = x * w1.y, x2 = x * w2.y;
+          s1 = fma3(make_float3(b0.x, b0.y, b0.z), make_float3(x1, x1, x1), s1);
+          s2 = fma3(make_float3(b0.x, b0.y, b0.z), make_float3(x2, x2, x2), s2);
+        };
+        if (has_lo) slope(-ssn, lo1, lo2);
+        if (has_hi) slope(ssn, hi1, hi2);
+#pragma unroll
+        for (int j = 0; j < GI; ++j) slope(sx[j], acc1[j], acc2[j]);
+        const float4* ka = L.ka + pr * KC;
+        const float* kb = L.kb + pr * KC;
+        for (int q = 0; q < cnt; ++q) {
+          const float4 kq = ka[q];
+          const float3 dB = make_float3(kq.z, kq.w, kb[q]);
+          auto add = [&](float d1, float d2, float3& s1, float3& s2) {
+            s1 = fma3(dB, make_float3(d1, d1, d1), s1);
+            s2 = fma3(dB, make_float3(d2, d2, d2), s2);
+          };
+          if (has_hi) {  // the arc |phi| < alpha
+            const uint32_t e = arc_entry(kq.x, Tr);
+            const float2 u1 = arc_ld<0>(e), u2 = arc_ld<1>(e);
+            add(2.0f * fmaf(kq.y, u1.x, ssn * u1.y), 2.0f * fmaf(kq.y, u2.x, ssn * u2.y), hi1, hi2);
+          }
+          if (has_lo) {  // the arc around pi: the row less |phi| < pi - alpha
+            const uint32_t e = arc_entry(float(NT) - kq.x, Tr);
+            const float2 u1 = arc_ld<0>(e), u2 = arc_ld<1>(e);
+            add(fmaf(kq.y, fmaf(-2.0f, u1.x, w1.x), -ssn * fmaf(-2.0f, u1.y, w1.y)),
+                fmaf(kq.y, fmaf(-2.0f, u2.x, w2.x), -ssn * fmaf(-2.0f, u2.y, w2.y)), lo1, lo2);
+          }
+#pragma unroll
+          for (int j = 0; j < GI; ++j) {
+            {
+              // the arc from phi_s - alpha to phi_s + alpha; sums below a
+              // negative angle are minus those below its opposite (sin: equal)
+              const float lo = phi[j] - kq.x, hi = phi[j] + kq.x;
+              const uint32_t ea = arc_entry(fabsf(lo), Tr), eb = arc_entry(hi, Tr);
+              const float sg = copysignf(1.0f, lo);
+              const float2 a1 = arc_ld<0>(ea), a2 = arc_ld<1>(ea), a3 = arc_ld<2>(ea);
+              const float2 b1 = arc_ld<0>(eb), b2 = arc_ld<1>(eb), b3 = arc_ld<2>(eb);
+              const float C1 = fmaf(-sg, a1.x, b1.x), X1 = fmaf(-sg, a1.y, b1.y), Y1 = b3.x - a3.x;
+              const float C2 = fmaf(-sg, a2.x, b2.x), X2 = fmaf(-sg, a2.y, b2.y), Y2 = b3.y - a3.y;
+              add(fmaf(sy[j], Y1, fmaf(sx[j], X1, kq.y * C1)), fmaf(sy[j], Y2, fmaf(sx[j], X2, kq.y * C2)), acc1[j],
+                  acc2[j]);
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  // --- results: phase weights folded, laid out in shared memory (T is no
+  // longer read), clamped texels copied from the ends, rows stored in runs of
+  // S columns
+  {
+    const float h0 = r - a.bottom;
+    const float rho_r = profile_density(a.ray_d, h0), rho_m = profile_density(a.mie_d, h0);
+    const float kmie = 3.0f / (8.0f * kPiF) * (1.0f - g * g) / (2.0f + g * g);
+    const float kray = 3.0f / (16.0f * kPiF);
+    const float3 A = make_float3(a.rayleigh[0] * rho_r * kray, a.rayleigh[1] * rho_r * kray, a.rayleigh[2] * rho_r * kray);
+    const float3 B = make_float3(a.mie_sca[0] * rho_m * kmie, a.mie_sca[1] * rho_m * kmie, a.mie_sca[2] * rho_m * kmie);
+    float* st = L.stage + c * kArcStage + lane;  // texel k, plane p at ((p nu + k) S) kArcStage
+    const int S33 = sh.S * kArcStage, P33 = n * S33;
+    auto put = [&](int k, float3 s1, float3 s2) {
+      s1 = s1 + com1;
+      s2 = s2 + com2;
+      float* o = st + k * S33;
+      o[0] = fmaf(A.x, s1.x, B.x * s2.x);
+      o[P33] = fmaf(A.y, s1.y, B.y * s2.y);
+      o[2 * P33] = fmaf(A.z, s1.z, B.z * s2.z);
+    };
+    if (has_col) {
+      if (has_lo) put(0, lo1, lo2);
+      if (has_hi) put(n - 1, hi1, hi2);
+#pragma unroll
+      for (int j = 0; j < GI; ++j)
+        if (j < kn) put(k0 + j, acc1[j], acc2[j]);
+    }
+    __syncthreads();
+    if (has_col) {
+#pragma unroll
+      for (int j = 0; j < GI; ++j) {
+        const int q = (cls >> (2 * j)) & 3;
+        if (j < kn && q) {
+          const float* from = st + (q == 1 ? 0 : n - 1) * S33;
+          float* o = st + (k0 + j) * S33;
+          o[0] = from[0];
+          o[P33] = from[P33];
+          o[2 * P33] = from[2 * P33];
+        }
+      }
+    }
+    __syncthreads();
+    // a warp stores 8 columns of 4 rows of one texel index and plane at a time
+    float* dens = a.dens + ((size_t)zi * a.sc_mu + y0) * 3 * a.Wd + s0;
+    const int cc = lane & 7, yl = lane >> 3;
+    for (int pk = warp; pk < 3 * n; pk += kArcWarps) {
+      const int p = pk >= n ? (pk >= 2 * n ? 2 : 1) : 0, k = pk - p * n;
+      if (cc < ns)
+        for (int yy = yl; yy < ny; yy += 4)
+          dens[((size_t)yy * 3 + p) * a.Wd + k * a.sc_mus + cc] = store_round(L.stage[(pk * sh.S + cc) * kArcStage + yy], a.f16);
+    }
+  }
+}
+
+// GI: the largest number of nu texels per thread in the launch (ends aside).
+// Density of orders >= 3 with the indirect irradiance of the order before.
+template <bool MX, int GI>
+__global__ void __launch_bounds__(kArcThreads, arc_ctas(GI)) k_density_arcs(LaunchArgs L) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  int seg, job, tile;
+  int taken = 0;
+  while (next_item(L, seg, job, tile, taken)) {
+    const DevAtmo& a = L.atm[job];
+    if (seg == 0) {
+      tile_density_arcs<MX, GI>(a, L.order, tile, L.arc_rows, smem);
+    } else {
+      const int kt = ir_items_kt(a.irr_n, a.sc_nu, a.W, a.ir_mus, false);
+      if (kt)
+        tile_indirect_rows<MX>(a, L.order, tile, kt, smem);
+      else
+        tile_indirect<MX>(a, L.order, tile, smem);
+    }
+  }
+}
+
+}  // namespace fb

@@ -77,7 +77,7 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Once per device, with that device current: the scratch address and every
 // pass kernel's dynamic shared-memory limit (the same kernels the builder sets
-// up: variants 0..5, of order 2 or not).
+// up: every variant, of order 2 or not).
 int setup_device(int dev, DeviceSetup** out) {
   std::lock_guard<std::mutex> g(g_setup_mu);
   DeviceSetup& d = g_setup[dev];
@@ -96,8 +96,9 @@ int setup_device(int dev, DeviceSetup** out) {
     for (int mode = 0; mode < 2; ++mode)
       for (int pass = 0; pass < 4; ++pass)
         for (int tpt : {1, 2})
-          for (int variant = 0; variant < 12; ++variant) {
-            const void* k = fb::kernel_for(mode == 1, pass, tpt, variant % 6, variant >= 6);
+          for (int variant = 0; variant < 2 * fb::kDensVariants; ++variant) {
+            const void* k =
+                fb::kernel_for(mode == 1, pass, tpt, variant % fb::kDensVariants, variant >= fb::kDensVariants);
             cudaFuncAttributes fa;
             if (cudaFuncGetAttributes(&fa, k) != cudaSuccess ||
                 cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -193,7 +194,7 @@ extern "C" int fb_atmosphere_build_noalloc(void* stream, const fb_params* p, voi
   // Each is checked and its grid decided here; launches without work items
   // (order 1 has none after the first two) are left out.
   std::vector<Launch> L;
-  int slot = 0;
+  int slot = 0, arc_rows = 0;
   auto add = [&](int pass, int order, std::vector<int> tiles, size_t smem, int tpt, int block,
                  int variant) -> int {
     const int k = slot++;
@@ -205,6 +206,7 @@ extern "C" int fb_atmosphere_build_noalloc(void* stream, const fb_params* p, voi
     l.args.atm = d_atm;
     l.args.nseg = (int)tiles.size();
     l.args.order = order;
+    l.args.arc_rows = arc_rows;
     l.args.counter = d_cnt + k;
     int total = 0;
     for (int sgi = 0; sgi < (int)tiles.size(); ++sgi) {
@@ -247,10 +249,19 @@ extern "C" int fb_atmosphere_build_noalloc(void* stream, const fb_params* p, voi
   const int ms_variant = fb::ms_block_variant(ms_block) >= 0 ? fb::ms_block_variant(ms_block)
                          : (ms_tpt == 1 && fb::ms_fixed_layout(d.W, d.sc_mus) ? 4 : 0);
   for (int n = 2; !rc && n <= d.order; ++n) {
+    if (n >= 3 && d.arcs) {
+      const fb::ArcShape sh = fb::arc_shape(d.sc_r, d.sc_mu, d.sc_mus, d.sc_nu);
+      size_t sm = 0;
+      arc_rows = fb::arc_launch_rows(std::vector<int>{0}, [&](int) -> const fb::DevAtmo& { return d; }, fb::arc_ctas(sh.gi), &sm);
+      sm = std::max(sm, fb::indirect_smem(d.irr_n, d.sc_nu, d.W, d.ir_mus, false));
+      rc = add(fb::kPassDensity, n, {sh.tiles, fb::tiles_indirect(d.ir_mus, d.ir_r, d.irr_n, d.sc_nu, d.W, false)}, sm, 1,
+               fb::kArcThreads, fb::arc_variant(sh.gi));
+    } else {
     const bool cl = fb::density_smem(d, n == 2, mixed, false) > (size_t)std::max(0, ds->smem_optin - 1024);
     const size_t sm = std::max(fb::density_smem(d, n == 2, mixed, cl), fb::indirect_smem(d.irr_n, d.sc_nu, d.W, d.ir_mus, n - 1 == 1));
     rc = add(fb::kPassDensity, n, {fb::tiles_density(d), fb::tiles_indirect(d.ir_mus, d.ir_r, d.irr_n, d.sc_nu, d.W, n - 1 == 1)}, sm, 1,
              fb::kDensThreads, cl ? fb::kDensClamped : 0);
+    }
     if (!rc)
       rc = add(fb::kPassMultiple, n, {fb::tiles_multiple(d.W, d.sc_mus, d.ms_steps, d.sc_mu, d.sc_r, ms_block)},
                fb::ms_smem(d.W, d.ms_steps, d.sc_mus, ms_block), ms_tpt, ms_block, ms_variant);

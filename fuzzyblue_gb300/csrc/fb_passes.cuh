@@ -25,6 +25,7 @@
 namespace fb {
 
 constexpr int kThreads = 256;
+constexpr int kIrMaxThreads = 256;      // threads of the CTAs that take indirect-irradiance row items
 constexpr int kMaxTexelsPerThread = 8;  // multiple scattering: W <= 2048
 constexpr int kMaxThetas = 32;          // density_samples <= 32
 constexpr int kMaxNuSlices = 66;        // scattering_nu_size <= 64 (+2 guard slices)
@@ -50,6 +51,7 @@ struct LaunchArgs {
   // work list is empty). A limit lets the block scheduler interleave CTAs of
   // other streams (by priority) between items; the grid then covers the work.
   int max_items;
+  int arc_rows;  // k_density_arcs: theta rows whose running sums are held at a time
 };
 
 // Takes the next work item of the launch for this CTA; `taken` counts the
@@ -329,7 +331,7 @@ template <bool MX> __device__ void tile_geometry(const DevAtmo& a, int tile) {
     const int row = k - a.W;
     const uint32_t y = (uint32_t)(row % a.sc_mu), z = (uint32_t)(row / a.sc_mu);
     RowGeo o;
-    o.pad = 0;
+    o.mu_lo = o.om_hi = o.om_lo = 0.f;
     if (!MX) {
       Geo32 G;
       G.init(a);
@@ -358,6 +360,9 @@ template <bool MX> __device__ void tile_geometry(const DevAtmo& a, int tile) {
       o.dist = (float)o.distd;
       o.one_m_mu2 = (1.0 - p.mu) * (1.0 + p.mu);
       o.mud = p.mu;
+      o.mu_lo = (float)(p.mu - (double)o.mu);
+      o.om_hi = (float)o.one_m_mu2;
+      o.om_lo = (float)(o.one_m_mu2 - (double)o.om_hi);
       o.rr = o.two_r_mu = o.r_mu = 0.f;
     }
     a.g_rows[row] = o;
@@ -1376,7 +1381,7 @@ __host__ __device__ inline int ir_per_item(int irr_n, int sc_nu) {
 __host__ __device__ inline size_t ir_rows_smem(int irr_n, int sc_nu, int W, bool one, int kt) {
   const size_t NT = irr_n / 2, NP = 2 * (size_t)irr_n, f = one ? 2 : 1;
   return align16(sizeof(float) * NT * NP) + align16(sizeof(float2) * NT) + align16(sizeof(float4) * W) +
-         align16(sizeof(float4) * (size_t)kt * (sc_nu + 2) * f) + sizeof(double) * 3 * kDensThreads;
+         align16(sizeof(float4) * (size_t)kt * (sc_nu + 2) * f) + sizeof(double) * 3 * kIrMaxThreads;
 }
 constexpr size_t kIrRowsSmem = 48 * 1024;  // no more than the density tiles' own shared memory
 __host__ __device__ inline int ir_rows_kt(int irr_n, int sc_nu, int W, int ir_mus) {
@@ -1740,6 +1745,12 @@ __global__ void __launch_bounds__(kDensThreads, V == 0 ? 4 : (V == 1 ? 3 : 5)) k
     }
   }
 }
+
+}  // namespace fb
+
+#include "fb_density_arcs.cuh"
+
+namespace fb {
 
 // ================================================== multiple scattering ===
 // multiple_scattering.comp:9-93. Every texel of a row shares the ray (r, mu)
@@ -2204,5 +2215,10 @@ __host__ __device__ inline size_t density_smem(const DevAtmo& a, bool two, bool 
 // Density variants: the occupancy variant (0..2), plus kDensClamped for the
 // clamped interval tables.
 constexpr int kDensClamped = 3;
+// Orders >= 3 by arcs: variants kDensArcs + 0, 1, 2 for at most 2, 6 and
+// kArcMaxGroup nu texels per thread besides the ends.
+constexpr int kDensArcs = 2 * kDensClamped;
+constexpr int kDensVariants = kDensArcs + 3;
+__host__ __device__ inline int arc_variant(int gi) { return kDensArcs + (gi <= 2 ? 0 : (gi <= 6 ? 1 : 2)); }
 
 }  // namespace fb

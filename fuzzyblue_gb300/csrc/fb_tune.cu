@@ -88,6 +88,10 @@ extern "C" int fb_builder_autotune(fb_builder* b, const fb_params* classes, uint
     e.sc_mus = (int)r.scattering_mu_s_size;
     e.sc_nu = (int)r.scattering_nu_size;
     e.precision = (int)p.precision;
+    // the tile shapes apply to order 2 alone where the later orders go by arcs
+    fb::DevAtmo d;
+    fbi::fill_atmo_record(d, p);
+    const int order = d.arcs ? 2 : 3;
     fbi::TuneEntry best = e;
     best.dens_ms = -1.0f;
     for (const Cand& cd : density_candidates(p)) {
@@ -100,7 +104,7 @@ extern "C" int fb_builder_autotune(fb_builder* b, const fb_params* classes, uint
           std::lock_guard<std::mutex> g(fbi::builder_mutex(b));
           fbi::tuning_set(fbi::builder_tuning(b), t);
         }
-        const float ms = time_launch(b, batchv, FB_KERNEL_DENSITY, 3, 2);
+        const float ms = time_launch(b, batchv, FB_KERNEL_DENSITY, order, 2);
         if (ms < 0) continue;  // a candidate that cannot launch here (e.g. its shared memory) is skipped
         if (best.dens_ms < 0 || ms < best.dens_ms) {
           best = t;
