@@ -608,14 +608,14 @@ void plan_group(Plan& P, const std::vector<DevAtmo>& A, const std::vector<int>& 
         const fb::ArcShape sh = fb::arc_shape(a.sc_r, a.sc_mu, a.sc_mus, a.sc_nu);
         gi = std::max(gi, sh.gi);
         t0.push_back(sh.tiles);
-        t1.push_back(fb::tiles_indirect(a.ir_mus, a.ir_r, a.irr_n, a.sc_nu, a.W, false));
+        t1.push_back(fb::tiles_indirect(a.ir_mus, a.ir_r, a.irr_n, a.sc_nu, false));
         D.texels += (uint64_t)a.W * a.sc_mu * a.sc_r + (uint64_t)a.ir_mus * a.ir_r;
       }
       D.block = fb::kArcThreads;
       D.variant = fb::arc_variant(gi);
       D.arc_rows = fb::arc_launch_rows(arcs, [&](int j) -> const DevAtmo& { return A[j]; }, fb::arc_ctas(gi), &D.smem);
       for (int j : arcs)
-        D.smem = std::max(D.smem, fb::indirect_smem(A[j].irr_n, A[j].sc_nu, A[j].W, A[j].ir_mus, false));
+        D.smem = std::max(D.smem, fb::indirect_smem(A[j].irr_n, A[j].sc_nu, A[j].W, false, D.block));
       add_segment(P, D, 0, arcs, t0);
       add_segment(P, D, 1, arcs, t1);
       D.nseg = 2;
@@ -632,9 +632,9 @@ void plan_group(Plan& P, const std::vector<DevAtmo>& A, const std::vector<int>& 
     for (int j : direct) {
       const DevAtmo& a = A[j];
       t0.push_back(fb::tiles_density(a));
-      t1.push_back(fb::tiles_indirect(a.ir_mus, a.ir_r, a.irr_n, a.sc_nu, a.W, n - 1 == 1));
+      t1.push_back(fb::tiles_indirect(a.ir_mus, a.ir_r, a.irr_n, a.sc_nu, n - 1 == 1));
       D.smem = std::max(D.smem, fb::density_smem(a, n == 2, mixed, cl));
-      D.smem = std::max(D.smem, fb::indirect_smem(a.irr_n, a.sc_nu, a.W, a.ir_mus, n - 1 == 1));
+      D.smem = std::max(D.smem, fb::indirect_smem(a.irr_n, a.sc_nu, a.W, n - 1 == 1, D.block));
       D.texels += (uint64_t)a.W * a.sc_mu * a.sc_r + (uint64_t)a.ir_mus * a.ir_r;
     }
     add_segment(P, D, 0, direct, t0);

@@ -17,9 +17,9 @@
 // arc. This is the sum over all directions, regrouped: a row costs as many
 // steps as it has knots (4-5 on average for 8 nu slices) instead of 32
 // directions. Measured against the direct sums (tile_density), density of order
-// 3: 16 default atmospheres 6.46 -> 2.25 ms, one of twice the size in every
-// dimension (16 nu slices) 6.58 -> 4.1 ms, one default atmosphere 0.461 -> 0.175
-// ms, with the same errors against FP64. Bound by the shared-memory pipe (76 %
+// 3 with its indirect irradiance: 16 default atmospheres 6.46 -> 1.98 ms, one of
+// twice the size in every dimension (16 nu slices) 6.58 -> 3.79 ms, one default
+// atmosphere 0.461 -> 0.156 ms, with the same errors against FP64. Bound by the shared-memory pipe (76 %
 // of its wavefronts; six 8-byte loads per texel and knot) and, between the
 // batches of theta rows, by the latency of building the next ones.
 //
@@ -536,11 +536,7 @@ __global__ void __launch_bounds__(kArcThreads, arc_ctas(GI)) k_density_arcs(Laun
     if (seg == 0) {
       tile_density_arcs<MX, GI>(a, L.order, tile, L.arc_rows, smem);
     } else {
-      const int kt = ir_items_kt(a.irr_n, a.sc_nu, a.W, a.ir_mus, false);
-      if (kt)
-        tile_indirect_rows<MX>(a, L.order, tile, kt, smem);
-      else
-        tile_indirect<MX>(a, L.order, tile, smem);
+      tile_indirect_arcs<MX>(a, L.order, tile, smem);
     }
   }
 }

@@ -253,13 +253,13 @@ extern "C" int fb_atmosphere_build_noalloc(void* stream, const fb_params* p, voi
       const fb::ArcShape sh = fb::arc_shape(d.sc_r, d.sc_mu, d.sc_mus, d.sc_nu);
       size_t sm = 0;
       arc_rows = fb::arc_launch_rows(std::vector<int>{0}, [&](int) -> const fb::DevAtmo& { return d; }, fb::arc_ctas(sh.gi), &sm);
-      sm = std::max(sm, fb::indirect_smem(d.irr_n, d.sc_nu, d.W, d.ir_mus, false));
-      rc = add(fb::kPassDensity, n, {sh.tiles, fb::tiles_indirect(d.ir_mus, d.ir_r, d.irr_n, d.sc_nu, d.W, false)}, sm, 1,
+      sm = std::max(sm, fb::indirect_smem(d.irr_n, d.sc_nu, d.W, false, fb::kArcThreads));
+      rc = add(fb::kPassDensity, n, {sh.tiles, fb::tiles_indirect(d.ir_mus, d.ir_r, d.irr_n, d.sc_nu, false)}, sm, 1,
                fb::kArcThreads, fb::arc_variant(sh.gi));
     } else {
     const bool cl = fb::density_smem(d, n == 2, mixed, false) > (size_t)std::max(0, ds->smem_optin - 1024);
-    const size_t sm = std::max(fb::density_smem(d, n == 2, mixed, cl), fb::indirect_smem(d.irr_n, d.sc_nu, d.W, d.ir_mus, n - 1 == 1));
-    rc = add(fb::kPassDensity, n, {fb::tiles_density(d), fb::tiles_indirect(d.ir_mus, d.ir_r, d.irr_n, d.sc_nu, d.W, n - 1 == 1)}, sm, 1,
+    const size_t sm = std::max(fb::density_smem(d, n == 2, mixed, cl), fb::indirect_smem(d.irr_n, d.sc_nu, d.W, n - 1 == 1, fb::kDensThreads));
+    rc = add(fb::kPassDensity, n, {fb::tiles_density(d), fb::tiles_indirect(d.ir_mus, d.ir_r, d.irr_n, d.sc_nu, n - 1 == 1)}, sm, 1,
              fb::kDensThreads, cl ? fb::kDensClamped : 0);
     }
     if (!rc)

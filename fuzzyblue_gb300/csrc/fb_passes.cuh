@@ -11,6 +11,7 @@
 //                    multiple-scattering samples (seg 2)     thread per (row, sample)
 //                    density r / theta records (segment 3)   thread per record
 //   k_density        scattering_density.comp (segment 0)     CTA per (r, mu_s, mu-chunk)
+//   k_density_arcs     the same for orders >= 3              CTA per (r, mu_s columns, 32 mu rows)
 //                    indirect_irradiance.comp (segment 1)    CTA per irradiance r row (up to 64 texels);
 //                                                            order 1: four texels, a warp each
 //   k_multiple       multiple_scattering.comp                CTA per (mu, r) row(s); variants 4
@@ -25,7 +26,6 @@
 namespace fb {
 
 constexpr int kThreads = 256;
-constexpr int kIrMaxThreads = 256;      // threads of the CTAs that take indirect-irradiance row items
 constexpr int kMaxTexelsPerThread = 8;  // multiple scattering: W <= 2048
 constexpr int kMaxThetas = 32;          // density_samples <= 32
 constexpr int kMaxNuSlices = 66;        // scattering_nu_size <= 64 (+2 guard slices)
@@ -1350,67 +1350,71 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
 }
 
 // ================================================== indirect irradiance ===
-// indirect_irradiance.comp:10-74. A work item is K irradiance texels (K = 4
-// where shared memory allows, see ir_per_item), one warp per texel: the warp
-// reduces the order's table to P[theta][nu slice] at its texel's (r, mu_s),
-// its lanes split the 16 x 64 directions, and a warp shuffle sums them. The
-// CTA first tabulates the directions once for its K texels: per direction
-// cos phi sin theta, per theta row cos theta and the solid angle (the same
-// float arithmetic as evaluating them per direction).
+// indirect_irradiance.comp:10-74. Order 1 (the single-scattering Rayleigh and
+// Mie tables with their phase functions, launch of order 2): a work item is K
+// irradiance texels (K = 4 where shared memory allows, see ir_per_item), one
+// warp per texel: the warp reduces the tables to P[theta][nu slice] at its
+// texel's (r, mu_s), its lanes split the 16 x 64 directions, and a warp
+// shuffle sums them. The CTA first tabulates the directions once for its K
+// texels: per direction cos phi sin theta, per theta row cos theta and the
+// solid angle (the same float arithmetic as evaluating them per direction).
+// Later orders: tile_indirect_arcs.
 constexpr int kIrMaxPerItem = 4;  // texels per item: one per warp of a kDensThreads CTA
 constexpr size_t kIrItemSmem = 64 * 1024;
-__host__ __device__ inline size_t indirect_smem_k(int irr_n, int sc_nu, bool one, int k) {
+__host__ __device__ inline size_t indirect_smem_k(int irr_n, int sc_nu, int k) {
   const size_t NT = irr_n / 2, NP = 2 * (size_t)irr_n;
   return align16(sizeof(float) * NT * NP) + align16(sizeof(float2) * NT) +
-         (size_t)k * sizeof(float4) * NT * (sc_nu + 2) * (one ? 2 : 1);
+         (size_t)k * sizeof(float4) * NT * (sc_nu + 2) * 2;
 }
-// Texels per item: 4, 2 or 1, the most whose tables fit in kIrItemSmem (the
-// order-1 layout, the larger one, decides for every order).
+// Texels per item: 4, 2 or 1, the most whose tables fit in kIrItemSmem.
 __host__ __device__ inline int ir_per_item(int irr_n, int sc_nu) {
   int k = kIrMaxPerItem;
-  while (k > 1 && indirect_smem_k(irr_n, sc_nu, true, k) > kIrItemSmem) k >>= 1;
+  while (k > 1 && indirect_smem_k(irr_n, sc_nu, k) > kIrItemSmem) k >>= 1;
   return k;
 }
-// Row items (tile_indirect_rows): an item is up to KT irradiance texels of one
-// irradiance r row. Shared memory: the direction table, the table blended in
-// (mu, r) for one theta row over every x (B; order 1 blends the Rayleigh and
-// Mie tables through it in turn), the texels' slice entries of that theta row
-// (P, per table) and every thread's FP64 partial sums. KT is the largest of
-// 64, 32, 16 whose layout fits in kIrRowsSmem (the order-1 layout, the larger,
-// decides); 0 selects the per-texel items.
-__host__ __device__ inline size_t ir_rows_smem(int irr_n, int sc_nu, int W, bool one, int kt) {
-  const size_t NT = irr_n / 2, NP = 2 * (size_t)irr_n, f = one ? 2 : 1;
-  return align16(sizeof(float) * NT * NP) + align16(sizeof(float2) * NT) + align16(sizeof(float4) * W) +
-         align16(sizeof(float4) * (size_t)kt * (sc_nu + 2) * f) + sizeof(double) * 3 * kIrMaxThreads;
+// Arc items: up to kIrArcTexels texels of one irradiance r row, the theta rows
+// split over groups of warps, each with one theta row's table in shared memory
+// (as many groups as kIrArcSmem holds rows of W texels, at least one: W <= 2048).
+constexpr int kIrArcTexels = 64;
+constexpr size_t kIrArcSmem = 48 * 1024;
+__host__ __device__ inline int ir_arc_groups(int W, int threads) {
+  int g = threads / 32;
+  while (g > 1 && sizeof(float4) * (size_t)W * g > kIrArcSmem) g >>= 1;
+  return g;
 }
-constexpr size_t kIrRowsSmem = 48 * 1024;  // no more than the density tiles' own shared memory
-__host__ __device__ inline int ir_rows_kt(int irr_n, int sc_nu, int W, int ir_mus) {
-  for (int kt = 64; kt >= 16; kt >>= 1)
-    if (ir_rows_smem(irr_n, sc_nu, W, true, kt) <= kIrRowsSmem) return kt < ir_mus ? kt : ir_mus;
-  return 0;
+__host__ __device__ inline size_t ir_arc_smem(int irr_n, int W, int threads) {
+  const size_t rows = sizeof(float4) * (size_t)W * ir_arc_groups(W, threads);
+  const size_t sums = sizeof(double) * 3 * kIrArcTexels * (threads / 32);  // in the place of the rows
+  return align16(sizeof(float) * (irr_n + 1)) + (rows > sums ? rows : sums);
 }
-// Row items integrate orders >= 2 (the multiple-scattering table); order 1
-// (the Rayleigh and Mie tables with their phase functions) keeps the items of
-// up to four texels, which measured faster there (173.3 against 175.3 ms per
-// order-2 density launch of 256 default atmospheres).
-__host__ __device__ inline int ir_items_kt(int irr_n, int sc_nu, int W, int ir_mus, bool one) {
-  return one ? 0 : ir_rows_kt(irr_n, sc_nu, W, ir_mus);
+__host__ __device__ inline size_t indirect_smem(int irr_n, int sc_nu, int W, bool one, int threads) {
+  return one ? indirect_smem_k(irr_n, sc_nu, ir_per_item(irr_n, sc_nu)) : ir_arc_smem(irr_n, W, threads);
 }
-__host__ __device__ inline size_t indirect_smem(int irr_n, int sc_nu, int W, int ir_mus, bool one) {
-  const int kt = ir_items_kt(irr_n, sc_nu, W, ir_mus, one);
-  return kt ? ir_rows_smem(irr_n, sc_nu, W, one, kt) : indirect_smem_k(irr_n, sc_nu, one, ir_per_item(irr_n, sc_nu));
-}
-__host__ __device__ inline int tiles_indirect(int ir_mus, int ir_r, int irr_n, int sc_nu, int W, bool one) {
-  const int kt = ir_items_kt(irr_n, sc_nu, W, ir_mus, one);
-  if (kt) return ir_r * ((ir_mus + kt - 1) / kt);
+__host__ __device__ inline int tiles_indirect(int ir_mus, int ir_r, int irr_n, int sc_nu, bool one) {
+  if (!one) return ir_r * ((ir_mus + kIrArcTexels - 1) / kIrArcTexels);
   const int k = ir_per_item(irr_n, sc_nu);
   return (ir_mus * ir_r + k - 1) / k;
 }
 
+// Irradiance of one texel: the order's own table and the final one.
+template <bool MX>
+__device__ __forceinline__ void store_irradiance(const DevAtmo& a, int order, int t, double tx, double ty, double tz) {
+  const float3 res = make_float3((float)tx, (float)ty, (float)tz);
+  a.dirr[(order + 1) & 1][t] = make_float4(res.x, res.y, res.z, 0.f);
+  if (!MX) {
+    const float4 old = a.ir[t];
+    a.ir[t] = make_float4(res.x + old.x, res.y + old.y, res.z + old.z, 0.f + old.w);
+  } else {
+    double* acc3 = a.ir_acc + 3 * (size_t)t;
+    acc3[0] += tx;
+    acc3[1] += ty;
+    acc3[2] += tz;
+    a.ir[t] = make_float4((float)acc3[0], (float)acc3[1], (float)acc3[2], 0.f);
+  }
+}
+
 template <bool MX>
 __device__ void tile_indirect(const DevAtmo& a, int order, int tile, unsigned char* smem) {
-  const int ord = order - 1;  // order integrated (the push constant order-1)
-  const bool one = ord == 1;
   const int NT = a.irr_n / 2, NP = 2 * a.irr_n;
   const int NNU = a.sc_nu, NK = NNU + 2;
   const int K = ir_per_item(a.irr_n, a.sc_nu);
@@ -1428,7 +1432,7 @@ __device__ void tile_indirect(const DevAtmo& a, int order, int tile, unsigned ch
   const int t = tile * K + warp;
   const bool active = warp < K && t < a.ir_mus * a.ir_r;
   const int PS = NT * NK;  // entries of one table
-  float4* P = Pall + (size_t)(warp < K ? warp : 0) * PS * (one ? 2 : 1);
+  float4* P = Pall + (size_t)(warp < K ? warp : 0) * PS * 2;
   const int i = t % a.ir_mus, j = t / a.ir_mus;
   float r = 0.f, mu_s = 0.f, u_ms = 0.f;
   Axis az;
@@ -1450,7 +1454,6 @@ __device__ void tile_indirect(const DevAtmo& a, int order, int tile, unsigned ch
       az = bounded_axis(z.az, a.sc_r);
       mu_s = a.g_irmus[i];
     }
-    const float4* src0 = one ? a.dr : a.dms;
     for (int k = lane; k < PS; k += 32) {
       const int l = k / NK, sl = k % NK;
       Axis ay, ax;
@@ -1464,12 +1467,9 @@ __device__ void tile_indirect(const DevAtmo& a, int order, int tile, unsigned ch
         ay = bounded_axis(a.g_iry[j * NT + l], a.sc_mu);
         ax = bounded_axis(a.g_irx[i * NK + sl], a.W);
       }
-      const float3 v = fetch3(src0, a.W, a.sc_mu, ax, ay, az);
+      const float3 v = fetch3(a.dr, a.W, a.sc_mu, ax, ay, az), m = fetch3(a.dm, a.W, a.sc_mu, ax, ay, az);
       P[k] = make_float4(v.x, v.y, v.z, 0.f);
-      if (one) {
-        const float3 m = fetch3(a.dm, a.W, a.sc_mu, ax, ay, az);
-        P[PS + k] = make_float4(m.x, m.y, m.z, 0.f);
-      }
+      P[PS + k] = make_float4(m.x, m.y, m.z, 0.f);
     }
   }
   __syncthreads();
@@ -1497,22 +1497,15 @@ __device__ void tile_indirect(const DevAtmo& a, int order, int tile, unsigned ch
       const float lf = tcx - fk;
       fk = fminf(fmaxf(fk, -1.0f), float(NNU - 1));
       const int ks = (int)fk + 1;
+      const float4* Ml = Pl + PS;
+      const float4 r0 = Pl[ks], r1 = Pl[ks + 1], m0 = Ml[ks], m1 = Ml[ks + 1];
+      const float pr = kray * (1.0f + nu * nu);
+      const float rs = rsqrt_pos(g1 - g2 * nu);
+      const float pm = kmie * (1.0f + nu * nu) * (rs * rs * rs);
       float3 L;
-      if (one) {
-        const float4* Ml = Pl + PS;
-        const float4 r0 = Pl[ks], r1 = Pl[ks + 1], m0 = Ml[ks], m1 = Ml[ks + 1];
-        const float pr = kray * (1.0f + nu * nu);
-        const float rs = rsqrt_pos(g1 - g2 * nu);
-        const float pm = kmie * (1.0f + nu * nu) * (rs * rs * rs);
-        L.x = fmaf(r1.x - r0.x, lf, r0.x) * pr + fmaf(m1.x - m0.x, lf, m0.x) * pm;
-        L.y = fmaf(r1.y - r0.y, lf, r0.y) * pr + fmaf(m1.y - m0.y, lf, m0.y) * pm;
-        L.z = fmaf(r1.z - r0.z, lf, r0.z) * pr + fmaf(m1.z - m0.z, lf, m0.z) * pm;
-      } else {
-        const float4 r0 = Pl[ks], r1 = Pl[ks + 1];
-        L.x = fmaf(r1.x - r0.x, lf, r0.x);
-        L.y = fmaf(r1.y - r0.y, lf, r0.y);
-        L.z = fmaf(r1.z - r0.z, lf, r0.z);
-      }
+      L.x = fmaf(r1.x - r0.x, lf, r0.x) * pr + fmaf(m1.x - m0.x, lf, m0.x) * pm;
+      L.y = fmaf(r1.y - r0.y, lf, r0.y) * pr + fmaf(m1.y - m0.y, lf, m0.y) * pm;
+      L.z = fmaf(r1.z - r0.z, lf, r0.z) * pr + fmaf(m1.z - m0.z, lf, m0.z) * pm;
       const float3 v = L * ct * dom;
       part.x += v.x;
       part.y += v.y;
@@ -1531,193 +1524,165 @@ __device__ void tile_indirect(const DevAtmo& a, int order, int tile, unsigned ch
   const double ty = warp_sum((double)acc.s.y - (double)acc.c.y);
   const double tz = warp_sum((double)acc.s.z - (double)acc.c.z);
   if (lane == 0) {
-    const float3 res = make_float3((float)tx, (float)ty, (float)tz);
-    a.dirr[(order + 1) & 1][t] = make_float4(res.x, res.y, res.z, 0.f);
-    if (!MX) {
-      const float4 old = a.ir[t];
-      a.ir[t] = make_float4(res.x + old.x, res.y + old.y, res.z + old.z, 0.f + old.w);
-    } else {
-      double* acc3 = a.ir_acc + 3 * (size_t)t;
-      acc3[0] += tx;
-      acc3[1] += ty;
-      acc3[2] += tz;
-      a.ir[t] = make_float4((float)acc3[0], (float)acc3[1], (float)acc3[2], 0.f);
-    }
+    store_irradiance<MX>(a, order, t, tx, ty, tz);
   }
 }
 
-// Row items: KT irradiance texels of one irradiance r row. For each theta row
-// the CTA first blends the order's table in (mu, r) at that row's lookup
-// position for every x of the packed table (B; coalesced loads, each table
-// row read once for the item), then every texel's slice entries are linear
-// interpolations of B in x (P), then the texels' directions of that theta row
-// are summed. The interpolation is the same trilinear one (blended in y and
-// z, then in x). Each texel's directions are split over nth / KT threads
-// whose FP64 partial sums meet in shared memory.
+// Orders >= 2 of the integral: on a theta row the radiance is piecewise linear
+// in the position t = (nu_size - 1) / 2 (nu + 1) = base + s cos phi of a
+// direction's sun angle (omega_s lies at phi = 0), so the row's directions are
+// summed as a line and arcs, as the density's (fb_density_arcs.cuh), here with
+// equal weights: an arc |phi| < alpha holds 2 i directions whose cosines sum to
+// sin(i dphi) / sin(dphi / 2), with i the number of half-circle directions below
+// alpha. Per theta row a group of warps first blends the table in (mu, r) at the
+// row's lookup position for every x of the packed table (coalesced loads), then
+// every texel interpolates the slices its row spans from it. The groups take the
+// theta rows in turn, so an item's latency is two or four rows and not 16: the
+// item of 64 texels over 64 directions per row that this replaced took 75 us,
+// which was the whole density launch of small tables (order 3 of one atmosphere
+// of the smoke sizes 76 -> 29 us; of 20 half-class atmospheres 210 -> 136 us).
 template <bool MX>
-__device__ void tile_indirect_rows(const DevAtmo& a, int order, int tile, int KT, unsigned char* smem) {
-  const int ord = order - 1;  // order integrated (the push constant order-1)
-  const bool one = ord == 1;
-  const int NT = a.irr_n / 2, NP = 2 * a.irr_n;
-  const int NNU = a.sc_nu, NK = NNU + 2, W = a.W;
+__device__ void tile_indirect_arcs(const DevAtmo& a, int order, int tile, unsigned char* smem) {
+  const int NT = a.irr_n / 2, NH = a.irr_n, n = a.sc_nu, W = a.W;
   const int tid = threadIdx.x, nth = blockDim.x;
-  const int segs = (a.ir_mus + KT - 1) / KT;
-  const int j = tile / segs, i0 = (tile % segs) * KT;
-  const int nt = min(KT, a.ir_mus - i0);
-  float* Dcx = (float*)smem;                                          // NT * NP: cos phi sin theta
-  float2* Drow = (float2*)(smem + align16(sizeof(float) * NT * NP));  // NT: (cos theta, d omega)
-  float4* B = (float4*)((unsigned char*)Drow + align16(sizeof(float2) * NT));  // W
-  float4* P = (float4*)((unsigned char*)B + align16(sizeof(float4) * W));        // KT * NK (x2 for order 1)
-  double* X = (double*)((unsigned char*)P + align16(sizeof(float4) * (size_t)KT * NK * (one ? 2 : 1)));
+  const int segs = (a.ir_mus + kIrArcTexels - 1) / kIrArcTexels;
+  const int j = tile / segs, i0 = (tile % segs) * kIrArcTexels;
+  const int nt = min(kIrArcTexels, a.ir_mus - i0);
+  float* cs = (float*)smem;  // NH + 1: the sum of an arc's cosines
+  float4* Ball = (float4*)(smem + align16(sizeof(float) * (NH + 1)));
+  double* X = (double*)Ball;
+  const int NG = ir_arc_groups(W, nth), gth = nth / NG, grp = tid / gth, gt = tid - grp * gth;
+  float4* B = Ball + (size_t)grp * W;
   const float dthetaf = kPiF / float(a.irr_n), dphif = kPiF / float(a.irr_n);
-  for (int k = tid; k < NT * NP; k += nth) {
-    const int l = k / NP, m = k % NP;
-    const float theta = (float(l) + 0.5f) * dthetaf, phi = (float(m) + 0.5f) * dphif;
-    Dcx[k] = cosf(phi) * sinf(theta);
-    if (m == 0) Drow[l] = make_float2(cosf(theta), dthetaf * dphif * sinf(theta));
-  }
-  // this irradiance row and the thread's texel (t) and share of its directions (h of H)
-  const int H = nth / KT, t = tid % KT, h = tid / KT;
-  const bool active = t < nt && h < H;
-  const int i = i0 + (t < nt ? t : 0);
-  float r = 0.f, mu_s, u_ms = 0.f;
+  for (int k = tid; k <= NH; k += nth) cs[k] = sinf(float(k) * dphif) / sinf(0.5f * dphif);
+  float r = 0.f;
   Axis az;
   if (!MX) {
     Geo32 G;
     G.init(a);
-    const float x_mu_s = float(i) / float(a.ir_mus - 1), x_r = float(j) / float(a.ir_r - 1);
+    const float x_r = float(j) / float(a.ir_r - 1);
     r = G.R + x_r * (G.T - G.R);
-    mu_s = clamp_cosine(2.0f * x_mu_s - 1.0f);
     az = make_axis(G.u_r(a, r), a.sc_r);
-    u_ms = G.u_mu_s(a, mu_s);
   } else {
     const IrZ z = a.g_irz[j];
     r = z.r;
     az = bounded_axis(z.az, a.sc_r);
-    mu_s = a.g_irmus[i];
   }
-  const float4* src0 = one ? a.dr : a.dms;
-  const float sxs = sqrtf(1.0f - mu_s * mu_s);
-  const float g = a.g;
-  const float kmie = 3.0f / (8.0f * kPiF) * (1.0f - g * g) / (2.0f + g * g);
-  const float kray = 3.0f / (16.0f * kPiF);
-  const float g1 = 1.0f + g * g, g2 = 2.0f * g;
-  const float fnu = float(NNU - 1);
-  const int PS = KT * NK;
-  Kahan3 acc;
-  acc.init();
-  for (int l = 0; l < NT; ++l) {
-    // B: the table at this theta row's (mu, r) position, every x
-    Axis ay;
+  // a thread's texels: gt and gt + gth of the item
+  constexpr int TX = kIrArcTexels / 32;
+  float mu_s[TX], u_ms[TX];
+  Axis ax[TX];
+  Kahan3 acc[TX];
+#pragma unroll
+  for (int q = 0; q < TX; ++q) {
+    acc[q].init();
+    const int i = i0 + min(gt + q * gth, nt - 1);
     if (!MX) {
       Geo32 G;
       G.init(a);
-      ay = make_axis(G.u_mu(a, r, cosf((float(l) + 0.5f) * dthetaf), false), a.sc_mu);
+      mu_s[q] = clamp_cosine(2.0f * (float(i) / float(a.ir_mus - 1)) - 1.0f);
+      u_ms[q] = G.u_mu_s(a, mu_s[q]);
     } else {
-      ay = bounded_axis(a.g_iry[j * NT + l], a.sc_mu);
+      mu_s[q] = a.g_irmus[i];
+      ax[q] = bounded_axis(a.g_irx[i * (n + 2) + 1], W);  // nu slice 0
+      u_ms[q] = 0.f;
     }
-    const float w00 = (1.0f - ay.f) * (1.0f - az.f), w10 = ay.f * (1.0f - az.f);
-    const float w01 = (1.0f - ay.f) * az.f, w11 = ay.f * az.f;
-    const size_t r00 = ((size_t)az.i0 * a.sc_mu + ay.i0) * W, r10 = ((size_t)az.i0 * a.sc_mu + ay.i1) * W;
-    const size_t r01 = ((size_t)az.i1 * a.sc_mu + ay.i0) * W, r11 = ((size_t)az.i1 * a.sc_mu + ay.i1) * W;
-    for (int tab = 0; tab < (one ? 2 : 1); ++tab) {
-      const float4* T = tab ? a.dm : src0;
-      for (int x = tid; x < W; x += nth) {
-        const float4 p00 = ld4(T + r00 + x), p10 = ld4(T + r10 + x), p01 = ld4(T + r01 + x), p11 = ld4(T + r11 + x);
+  }
+  const float hP = 0.5f * float(n - 1);
+  for (int l0 = 0; l0 < NT; l0 += NG) {
+    const int l = l0 + grp;
+    if (l < NT) {  // B: the table at this theta row's (mu, r) position, every x
+      Axis ay;
+      if (!MX) {
+        Geo32 G;
+        G.init(a);
+        ay = make_axis(G.u_mu(a, r, cosf((float(l) + 0.5f) * dthetaf), false), a.sc_mu);
+      } else {
+        ay = bounded_axis(a.g_iry[j * NT + l], a.sc_mu);
+      }
+      const float w00 = (1.0f - ay.f) * (1.0f - az.f), w10 = ay.f * (1.0f - az.f);
+      const float w01 = (1.0f - ay.f) * az.f, w11 = ay.f * az.f;
+      const float4* T00 = a.dms + ((size_t)az.i0 * a.sc_mu + ay.i0) * W;
+      const float4* T10 = a.dms + ((size_t)az.i0 * a.sc_mu + ay.i1) * W;
+      const float4* T01 = a.dms + ((size_t)az.i1 * a.sc_mu + ay.i0) * W;
+      const float4* T11 = a.dms + ((size_t)az.i1 * a.sc_mu + ay.i1) * W;
+#pragma unroll 4
+      for (int x = gt; x < W; x += gth) {
+        const float4 p00 = ld4(T00 + x), p10 = ld4(T10 + x), p01 = ld4(T01 + x), p11 = ld4(T11 + x);
         B[x] = make_float4(fmaf(w11, p11.x, fmaf(w01, p01.x, fmaf(w10, p10.x, w00 * p00.x))),
                            fmaf(w11, p11.y, fmaf(w01, p01.y, fmaf(w10, p10.y, w00 * p00.y))),
                            fmaf(w11, p11.z, fmaf(w01, p01.z, fmaf(w10, p10.z, w00 * p00.z))), 0.f);
       }
-      __syncthreads();
-      // P: each texel's entries of the nu slices -1 .. nu_size at its mu_s
-      float4* Pt = P + tab * PS;
-      for (int e = tid; e < nt * NK; e += nth) {
-        const int t2 = e / NK, sl = e - t2 * NK;
-        Axis ax;
-        if (!MX) {
-          Geo32 G;
-          G.init(a);
-          const float ms2 = clamp_cosine(2.0f * (float(i0 + t2) / float(a.ir_mus - 1)) - 1.0f);
-          ax = make_axis((float(sl - 1) + G.u_mu_s(a, ms2)) / float(NNU), a.W);
-        } else {
-          ax = bounded_axis(a.g_irx[(i0 + t2) * NK + sl], a.W);
-        }
-        const float4 b0 = B[ax.i0], b1 = B[ax.i1];
-        const float f0 = 1.0f - ax.f;
-        Pt[e] = make_float4(fmaf(ax.f, b1.x, f0 * b0.x), fmaf(ax.f, b1.y, f0 * b0.y), fmaf(ax.f, b1.z, f0 * b0.z), 0.f);
-      }
-      __syncthreads();
     }
-    if (active) {
-      const float2 row = Drow[l];
-      const float ct = row.x, dom = row.y;
-      const float4* Pl = P + t * NK;
-      float3 part = make_float3(0.f, 0.f, 0.f);
-      for (int m = h; m < NP; m += H) {
-        // nu = dot(omega, omega_s) with omega_s = (sqrt(1 - mu_s^2), 0, mu_s)
-        const float nu = Dcx[l * NP + m] * sxs + ct * mu_s;
-        const float tcx = (nu + 1.0f) / 2.0f * fnu;
-        float fk = floorf(tcx);
-        const float lf = tcx - fk;
-        fk = fminf(fmaxf(fk, -1.0f), float(NNU - 1));
-        const int ks = (int)fk + 1;
-        float3 L;
-        if (one) {
-          const float4* Ml = Pl + PS;
-          const float4 r0 = Pl[ks], r1 = Pl[ks + 1], m0 = Ml[ks], m1 = Ml[ks + 1];
-          const float pr = kray * (1.0f + nu * nu);
-          const float rs = rsqrt_pos(g1 - g2 * nu);
-          const float pm = kmie * (1.0f + nu * nu) * (rs * rs * rs);
-          L.x = fmaf(r1.x - r0.x, lf, r0.x) * pr + fmaf(m1.x - m0.x, lf, m0.x) * pm;
-          L.y = fmaf(r1.y - r0.y, lf, r0.y) * pr + fmaf(m1.y - m0.y, lf, m0.y) * pm;
-          L.z = fmaf(r1.z - r0.z, lf, r0.z) * pr + fmaf(m1.z - m0.z, lf, m0.z) * pm;
-        } else {
-          const float4 r0 = Pl[ks], r1 = Pl[ks + 1];
-          L.x = fmaf(r1.x - r0.x, lf, r0.x);
-          L.y = fmaf(r1.y - r0.y, lf, r0.y);
-          L.z = fmaf(r1.z - r0.z, lf, r0.z);
+    __syncthreads();
+    if (l < NT) {
+      const float theta = (float(l) + 0.5f) * dthetaf, ct = cosf(theta), st = sinf(theta);
+      const float weight = ct * (dthetaf * dphif * st);
+#pragma unroll
+      for (int q = 0; q < TX; ++q) {
+        if (gt + q * gth < nt) {
+          // the texel's entry of slice k
+          auto entry = [&](int k) {
+            Axis x;
+            if (!MX) {
+              x = make_axis((float(k) + u_ms[q]) / float(n), W);
+            } else {
+              x = ax[q];
+              x.i0 = min(x.i0 + k * a.sc_mus, W - 1);
+              x.i1 = min(x.i1 + k * a.sc_mus, W - 1);
+            }
+            const float4 b0 = B[x.i0], b1 = B[x.i1];
+            const float f0 = 1.0f - x.f;
+            return make_float3(fmaf(x.f, b1.x, f0 * b0.x), fmaf(x.f, b1.y, f0 * b0.y), fmaf(x.f, b1.z, f0 * b0.z));
+          };
+          const float m = mu_s[q];
+          const float base = hP * fmaf(ct, m, 1.0f), s = hP * st * sqrtf(1.0f - m * m);
+          const int klo = min(max((int)floorf(base - s), 0), n - 2), khi = min(max((int)floorf(base + s), klo), n - 2);
+          const float3 v0 = entry(klo);
+          float3 v1 = entry(klo + 1);
+          float3 b = make_float3(v1.x - v0.x, v1.y - v0.y, v1.z - v0.z);
+          // the lowest interval's line at the row's mean position
+          const float f = base - float(klo), np = float(2 * NH);
+          float3 sum = make_float3(np * fmaf(f, b.x, v0.x), np * fmaf(f, b.y, v0.y), np * fmaf(f, b.z, v0.z));
+          for (int k = klo + 1; k <= khi; ++k) {
+            const float3 v2 = entry(k + 1);
+            const float3 b2 = make_float3(v2.x - v1.x, v2.y - v1.y, v2.z - v1.z);
+            const float co = fminf(fmaxf((float(k) - base) / s, -1.0f), 1.0f);
+            const int i = min(max(__float2int_rn(acosf(co) * (float(NH) / kPiF)), 0), NH);
+            const float d = fmaf(base - float(k), float(2 * i), s * cs[i]);
+            sum.x = fmaf(b2.x - b.x, d, sum.x);
+            sum.y = fmaf(b2.y - b.y, d, sum.y);
+            sum.z = fmaf(b2.z - b.z, d, sum.z);
+            b = b2;
+            v1 = v2;
+          }
+          acc[q].add(sum * weight);
         }
-        const float3 v = L * ct * dom;
-        part.x += v.x;
-        part.y += v.y;
-        part.z += v.z;
-      }
-      if (!MX) {
-        acc.s.x += part.x;
-        acc.s.y += part.y;
-        acc.s.z += part.z;
-      } else {
-        acc.add(part);
       }
     }
-    __syncthreads();  // B and P are rebuilt for the next theta row
+    __syncthreads();  // B is rebuilt for the next theta rows
   }
-  // the texel's partial sums, in FP64
-  X[3 * tid] = (double)acc.s.x - (double)acc.c.x;
-  X[3 * tid + 1] = (double)acc.s.y - (double)acc.c.y;
-  X[3 * tid + 2] = (double)acc.s.z - (double)acc.c.z;
+  // the groups' sums of each texel, in FP64
+#pragma unroll
+  for (int q = 0; q < TX; ++q) {
+    const int t = gt + q * gth;
+    if (t < nt) {
+      double* o = X + 3 * (grp * kIrArcTexels + t);
+      o[0] = (double)acc[q].s.x - (double)acc[q].c.x;
+      o[1] = (double)acc[q].s.y - (double)acc[q].c.y;
+      o[2] = (double)acc[q].s.z - (double)acc[q].c.z;
+    }
+  }
   __syncthreads();
-  if (h == 0 && t < nt) {
+  if (tid < nt) {
     double tx = 0.0, ty = 0.0, tz = 0.0;
-    for (int q = 0; q < H; ++q) {
-      const int o = 3 * (q * KT + t);
-      tx += X[o];
-      ty += X[o + 1];
-      tz += X[o + 2];
+    for (int q = 0; q < NG; ++q) {
+      const double* o = X + 3 * (q * kIrArcTexels + tid);
+      tx += o[0];
+      ty += o[1];
+      tz += o[2];
     }
-    const int tt = j * a.ir_mus + i;
-    const float3 res = make_float3((float)tx, (float)ty, (float)tz);
-    a.dirr[(order + 1) & 1][tt] = make_float4(res.x, res.y, res.z, 0.f);
-    if (!MX) {
-      const float4 old = a.ir[tt];
-      a.ir[tt] = make_float4(res.x + old.x, res.y + old.y, res.z + old.z, 0.f + old.w);
-    } else {
-      double* acc3 = a.ir_acc + 3 * (size_t)tt;
-      acc3[0] += tx;
-      acc3[1] += ty;
-      acc3[2] += tz;
-      a.ir[tt] = make_float4((float)acc3[0], (float)acc3[1], (float)acc3[2], 0.f);
-    }
+    store_irradiance<MX>(a, order, j * a.ir_mus + i0 + tid, tx, ty, tz);
   }
 }
 
@@ -1735,13 +1700,11 @@ __global__ void __launch_bounds__(kDensThreads, V == 0 ? 4 : (V == 1 ? 3 : 5)) k
       tile_density<MX, TWO, CL>(L.atm[job], L.order, tile, smem);
     } else {
       const DevAtmo& a = L.atm[job];
-      // order 2 (TWO) integrates order 1, which always takes the four-texel
-      // items: its kernel does not contain the row items
-      const int kt = TWO ? 0 : ir_items_kt(a.irr_n, a.sc_nu, a.W, a.ir_mus, false);
-      if (!TWO && kt)
-        tile_indirect_rows<MX>(a, L.order, tile, kt, smem);
-      else
+      // order 2 (TWO) integrates order 1, which has items of its own
+      if (TWO)
         tile_indirect<MX>(a, L.order, tile, smem);
+      else
+        tile_indirect_arcs<MX>(a, L.order, tile, smem);
     }
   }
 }
