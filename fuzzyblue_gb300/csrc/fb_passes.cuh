@@ -801,7 +801,7 @@ constexpr int kDensMaxGroup = 8;
 
 // Per-atmosphere tile shape of the density pass (host and device agree).
 struct DensShape {
-  int G;      // texels per thread (divides nu_size, <= kDensMaxGroup)
+  int G;      // texels per thread (<= kDensMaxGroup; the last group of a row may have fewer)
   int NG;     // nu groups per mu row
   int S;      // mu_s columns per tile
   int chunk;  // mu rows per tile
@@ -812,8 +812,8 @@ struct DensShape {
 __host__ __device__ inline DensShape dens_shape(int sc_r, int sc_mu, int sc_mus, int sc_nu, int S_req = 0,
                                                 int chunk_req = 0) {
   DensShape d;
-  d.G = (sc_nu % 8 == 0) ? 8 : (sc_nu % 4 == 0) ? 4 : (sc_nu % 2 == 0) ? 2 : 1;
-  d.NG = sc_nu / d.G;
+  d.NG = (sc_nu + kDensMaxGroup - 1) / kDensMaxGroup;
+  d.G = (sc_nu + d.NG - 1) / d.NG;
   const int per_col = sc_mu * d.NG;
   if (S_req > 0 && chunk_req > 0 && S_req * min(chunk_req, sc_mu) * d.NG <= kDensThreads) {
     d.S = min(S_req, sc_mus);
@@ -850,14 +850,20 @@ struct LerpRec {
   float2 b;
   float2 pad;
 };
-// Order 2: the Rayleigh and Mie intervals of the same nu position in one
-// 48-byte record, read as three 16-byte loads: a = (R value at 0, R slope x),
-// b = (R slope y, R slope z, M value at 0 x, y), c = (M value at 0 z, M slope).
-// Records 48 bytes apart also put the intervals 0-7 of a row on disjoint
-// banks for each 16-byte load.
-struct LerpRec2 {
-  float4 a, b, c;
-};
+// Order 2: the Rayleigh and Mie intervals of the same nu position, as lines in
+// nu itself: three 16-byte words (R value at nu = 0, R slope x), (R slope y, R
+// slope z, M value at 0 x, y), (M value at 0 z, M slope), each word in an array
+// of its own per theta row (dens2_slots records), so that eight neighbouring
+// intervals lie on disjoint banks and a record's address is one shift and add.
+//
+// The interval of nu is (nu_size - 1) / 2 nu - v_off rounded to an integer,
+// plus the first interval's; v_off (0 for an even nu_size, 1/2 for an odd one)
+// puts the intervals' borders halfway between integers. Shrunk by kDens2Shrink,
+// which is above the rounding of nu, the range [-1, 1] has exactly the
+// nu_size - 1 intervals. A direction within 2e-6 of a border may take the
+// neighbouring line, which meets its own there.
+constexpr float kDens2Shrink = 1.0f - 0x1p-19f;
+__host__ __device__ inline int dens2_slots(int sc_nu) { return sc_nu <= 8 ? 8 : (sc_nu <= 16 ? 16 : sc_nu); }
 
 // The density tile's interval tables have a power-of-two number of records,
 // addressed by k & (size - 1): intervals k >= 0 at position k, the interval
@@ -886,8 +892,11 @@ struct DensLayout {
   Axis* kax;        // S * NK: (column, nu slice) -> x axis
   float2* dir;      // NT * NT mirror pairs: (cos phi sin t, sin phi sin t) x (nu_size - 1) / 2
   float2* gw;       // NT: ground rows, the ground table position as a function of w: (A, B0)
-  LerpRec* P;       // S * NT * MK: nu intervals of the previous order (dens_mk); order 2:
-                    // LerpRec2 records of the Rayleigh and Mie tables
+  LerpRec* P;       // S * NT * MK: nu intervals of the previous order (dens_mk)
+  float4* P2;       // order 2, in its place: S * NT * 3 * dens2_slots words of the Rayleigh and Mie tables
+  float4* gl;       // order 2: S * NT * 2: the ground bounce of a row whose directions see one interval of the
+                    // ground row, as a line in nu: (value at 0, kind), (slope); kind 1: a line
+                    // (0 where the row meets no ground), 2: several intervals
   LerpRec* E;       // MKE: intervals of the ground irradiance row, the two sampler rows pre-blended (dens_mke)
   float* col_mus;   // S
   double* col_musd; // S (MIXED)
@@ -899,7 +908,8 @@ struct DensLayout {
 __host__ __device__ inline size_t dens_layout(unsigned char* base, int dens_n, int sc_nu, int ir_mus, int S,
                                               int chunk, bool two, bool mixed, bool cl, DensLayout* L) {
   const int NT = dens_n, NK = sc_nu + 2;
-  const size_t nP = (size_t)S * NT * dens_mk(sc_nu, cl);
+  const size_t p_bytes = two ? sizeof(float4) * S * NT * 3 * dens2_slots(sc_nu)
+                             : sizeof(LerpRec) * S * NT * dens_mk(sc_nu, cl);
   size_t o = 0;
   auto take = [&](size_t bytes) {
     size_t at = o;
@@ -908,7 +918,7 @@ __host__ __device__ inline size_t dens_layout(unsigned char* base, int dens_n, i
   };
   size_t o_th = take(sizeof(DensTheta) * NT), o_tay = take(sizeof(Axis) * NT), o_kax = take(sizeof(Axis) * S * NK);
   size_t o_dir = take(sizeof(float2) * NT * NT), o_gw = take(sizeof(float2) * NT);
-  size_t o_P = take((two ? sizeof(LerpRec2) : sizeof(LerpRec)) * nP), o_E = take(sizeof(LerpRec) * dens_mke(ir_mus, cl));
+  size_t o_P = take(p_bytes), o_gl = take(two ? sizeof(float4) * S * NT * 2 : 0), o_E = take(sizeof(LerpRec) * dens_mke(ir_mus, cl));
   size_t o_cm = take(sizeof(float) * S), o_cmd = take(sizeof(double) * S);
   size_t o_ymu = take(mixed ? sizeof(double2) * chunk : 0), o_nu = take(mixed ? sizeof(double) * sc_nu : 0);
   size_t o_acc = take(mixed ? sizeof(float) * kDensThreads * kDensMaxGroup * 6 : 0);
@@ -919,6 +929,8 @@ __host__ __device__ inline size_t dens_layout(unsigned char* base, int dens_n, i
     L->dir = (float2*)(base + o_dir);
     L->gw = (float2*)(base + o_gw);
     L->P = (LerpRec*)(base + o_P);
+    L->P2 = (float4*)(base + o_P);
+    L->gl = (float4*)(base + o_gl);
     L->E = (LerpRec*)(base + o_E);
     L->col_mus = (float*)(base + o_cm);
     L->col_musd = (double*)(base + o_cmd);
@@ -962,6 +974,11 @@ template <bool CL> __device__ __forceinline__ int line_pos(float w, int n) {
   return __float_as_int(y) & (n - 1);
 }
 
+// A compile-time integer as an argument of a lambda.
+template <int N> struct Int {
+  static constexpr int value = N;
+};
+
 // The directions of one theta row for the G texels of a thread (all sharing
 // r, mu and mu_s): incident radiance of order n - 1 from the reduced table
 // (scattering.h:139-179), plus for rows that meet the ground the ground
@@ -980,12 +997,11 @@ template <bool CL> __device__ __forceinline__ int line_pos(float w, int n) {
 struct DensRowConst {
   float mu, muh, mu_s, oxs;  // mu; mu_s (nu_size - 1) / 2; mu_s; sqrt(1 - mu^2) / ((nu_size - 1) / 2)
   float offP, gmus;          // (n - 1) / 2 - 1/2 of the nu table; hE (r / R) mu_s
-  float inv_h, c1;           // TWO: nu = w inv_h + c1
   int nP, nE;                 // records per nu table row and of the ground irradiance table
 };
 // GC: the texels per thread when known at compile time (kDensMaxGroup, the
 // classes with nu a multiple of 8), else 0 and G at run time.
-template <bool TWO, bool GROUND, bool CL, int GC>
+template <bool GROUND, bool CL, int GC>
 __device__ __forceinline__ void dens_row(const DensLayout& S, const DensTheta& t, int l, int NT,
                                          const LerpRec* __restrict__ Pl,
                                          const DensRowConst& q, const float (&sx)[kDensMaxGroup],
@@ -1012,24 +1028,9 @@ __device__ __forceinline__ void dens_row(const DensLayout& S, const DensTheta& t
         for (int side = 0; side < 2; ++side) {
           const float w = side ? base - dy : base + dy;
           const int k = line_pos<CL>(w, q.nP);
-          float3 inc;
-          if (!TWO) {
-            const float4 pa = Pl[k].a;
-            const float2 pb = Pl[k].b;
-            inc = make_float3(fmaf(pa.w, w, pa.x), fmaf(pb.x, w, pa.y), fmaf(pb.y, w, pa.z));
-          } else {
-            // R P_R(nu) + M P_M(nu) = (1 + nu^2) (kR R + kM (1 + g^2 - 2 g nu)^-3/2 M),
-            // the constants kR, kM folded into the tables
-            const LerpRec2& r2 = reinterpret_cast<const LerpRec2*>(Pl)[k];
-            const float4 ra = r2.a, rb = r2.b, rc = r2.c;
-            const float nu1 = fmaf(w, q.inv_h, q.c1);
-            const float t1 = fmaf(nu1, nu1, 1.0f);
-            const float rs = rsqrt_pos(fmaf(-pc.g2, nu1, pc.g1));
-            const float rs3 = rs * rs * rs;
-            inc.x = fmaf(fmaf(rc.y, w, rb.z), rs3, fmaf(ra.w, w, ra.x)) * t1;
-            inc.y = fmaf(fmaf(rc.z, w, rb.w), rs3, fmaf(rb.x, w, ra.y)) * t1;
-            inc.z = fmaf(fmaf(rc.w, w, rc.x), rs3, fmaf(rb.y, w, ra.z)) * t1;
-          }
+          const float4 pa = Pl[k].a;
+          const float2 pb = Pl[k].b;
+          float3 inc = make_float3(fmaf(pa.w, w, pa.x), fmaf(pb.x, w, pa.y), fmaf(pb.y, w, pa.z));
           if (GROUND) {
             // irradiance of order n - 2 where omega_i meets the ground
             const float we = fmaf(gA, w, gB);
@@ -1044,6 +1045,134 @@ __device__ __forceinline__ void dens_row(const DensLayout& S, const DensTheta& t
           acc[j].y = fmaf(inc.y, cf.y, acc[j].y);
           acc[j].z = fmaf(inc.z, cf.z, acc[j].z);
         }
+      }
+    }
+  }
+}
+
+// A 16-byte word of shared memory at a byte address and a constant offset.
+template <int OFF> __device__ __forceinline__ float4 ld_shared4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4 + %5];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr), "n"(OFF));
+  return v;
+}
+
+// The same for order 2, whose lookups read the single-scattering Rayleigh and
+// Mie tables with their phase functions: R P_R(nu) + M P_M(nu) = (1 + nu^2)
+// (kR R + kM (1 + g^2 - 2 g nu)^-3/2 M), the constants kR, kM folded into the
+// tables. Two things keep directions from being evaluated twice or at length:
+// the texels at nu = -1 and 1 (the clamp moves them into the plane of omega,
+// sun_y = 0) see both directions of a mirror pair alike, so their sums take one
+// of each and are doubled at the end; and the ground bounce of a row that sees
+// one interval of the ground row (GM = 1: five of six ground rows at the default
+// sizes) is a line in nu, so its sum follows from the row's sums of the phase
+// weights.
+// Against evaluating every direction of every texel, with a ground record each:
+// order 2 of 16 default atmospheres 10.66 -> 8.10 ms, of the double class 10.65
+// -> 9.2 ms, of 20 half-class ones 1.10 -> 0.77 ms. Bound by the shared-memory
+// pipe (82 % of its wavefronts, three 16-byte words per direction) and by issue
+// (71 %).
+// GC, SLC: the texels per thread and words per array where they are known (the
+// sizes of the table classes: 2, 4, 8 and 16 nu slices), else 0. ENDS: one group
+// per mu row, so that texels 0 and jh are the two ends; else lo1 and hi1 say
+// whether they are for the whole warp.
+struct Dens2Const {
+  float mu, mu_s, ox;     // ox: sqrt(1 - mu^2)
+  float scale, v_off;     // (nu_size - 1) / 2 kDens2Shrink
+  float g1, g2;           // 1 + g^2, 2 g
+  float gmus, hP;         // GM = 2: hE (r / R) mu_s, (nu_size - 1) / 2
+  int k0, slots, nE;      // the first interval's integer; words per array of a row; records of the ground table
+};
+template <int GM, bool CL, int GC, int SLC, bool ENDS>
+__device__ __forceinline__ void dens_row2(const DensLayout& S, const DensTheta& t, int l, int NT,
+                                          const float4* __restrict__ Pl, const float4* gl, const Dens2Const& q,
+                                          const float (&sx)[kDensMaxGroup], const float (&sy)[kDensMaxGroup], int Gr,
+                                          int jhr, bool lo1, bool hi1, const PhaseCoef& pc, float3 (&acc)[kDensMaxGroup]) {
+  const int G = GC ? GC : Gr, jh = GC ? GC - 1 : jhr, SL = SLC ? SLC : q.slots;
+  const float mus_ct = q.mu_s * t.cos_t, mu_ct = q.mu * t.cos_t;
+  const float2* dirl = S.dir + l * NT;
+  // the interval is in the low bits of the sum with 1.5 2^23, less the bits of
+  // that constant and of the first interval. (Through a shuffle, so that the
+  // assembler does not add these terms anew for each load. |nu| <= 3 whatever
+  // the tables hold, so that no lookup leaves shared memory.)
+  uint32_t Pk = (uint32_t)__cvta_generic_to_shared(Pl) - (uint32_t)(kRoundMagicBits - q.k0) * 16u;
+  Pk = __shfl_sync(__activemask(), Pk, threadIdx.x & 31);
+  float gA = 0.f, gB = 0.f;
+  if (GM == 2) {
+    const float2 g = S.gw[l];
+    gA = g.x * q.hP;
+    gB = fmaf(g.x, q.hP - 0.5f, g.y + q.gmus);
+  }
+  float3 SC = make_float3(0.f, 0.f, 0.f), SX = SC;
+  for (int m = 0; m < NT; ++m) {
+    const float2 d = dirl[m];
+    // phase functions of omega . omega_i, shared by the pair and the group
+    const float nu2 = fmaf(q.ox, d.x, mu_ct);
+    const float3 cf = pc.eval(nu2, t.domega);
+    if (GM == 1) {
+      SC = SC + cf;
+      SX = fma3(cf, make_float3(d.x, d.x, d.x), SX);
+    }
+#pragma unroll
+    for (int j = 0; j < kDensMaxGroup; ++j) {
+      if (j < G) {
+        const float base = fmaf(sx[j], d.x, mus_ct);
+        // the radiance from nu: inc (1 + nu^2), the factor apart
+        auto eval = [&](float nu, float3& inc, float& t1) {
+          // (the sizes compiled for are even: v_off is 0)
+          const float y = GC ? fmaf(nu, q.scale, kRoundMagic) : fmaf(nu, q.scale, -q.v_off) + kRoundMagic;
+          const uint32_t at = ((uint32_t)__float_as_int(y) << 4) + Pk;
+          const float4 ra = ld_shared4<0>(at), rb = SLC ? ld_shared4<SLC * 16>(at) : ld_shared4<0>(at + SL * 16);
+          const float4 rc = SLC ? ld_shared4<SLC * 32>(at) : ld_shared4<0>(at + SL * 32);
+          t1 = fmaf(nu, nu, 1.0f);
+          const float rs = rsqrt_pos(fmaf(-q.g2, nu, q.g1));
+          const float rs3 = rs * rs * rs;
+          inc.x = fmaf(fmaf(rc.y, nu, rb.z), rs3, fmaf(ra.w, nu, ra.x));
+          inc.y = fmaf(fmaf(rc.z, nu, rb.w), rs3, fmaf(rb.x, nu, ra.y));
+          inc.z = fmaf(fmaf(rc.w, nu, rc.x), rs3, fmaf(rb.y, nu, ra.z));
+        };
+        // direct irradiance where omega_i meets the ground
+        auto ground = [&](float nu, float3 inc) {
+          if (GM == 2) {
+            const float we = fmaf(gA, nu, gB);
+            const int e = line_pos<CL>(we, q.nE);
+            const float4 ea = S.E[e].a;
+            const float2 eb = S.E[e].b;
+            inc.x = fmaf(t.tgx, fmaf(ea.w, we, ea.x), inc.x);
+            inc.y = fmaf(t.tgy, fmaf(eb.x, we, ea.y), inc.y);
+            inc.z = fmaf(t.tgz, fmaf(eb.y, we, ea.z), inc.z);
+          }
+          return inc;
+        };
+        float3 inc;
+        float t1;
+        if ((j == 0 && (ENDS || lo1)) || (j == jh && (ENDS || hi1))) {
+          eval(base, inc, t1);
+          acc[j] = fma3(ground(base, inc * t1), cf, acc[j]);
+        } else {
+          // both directions of the pair before the weight: one FMA less per channel
+          float3 inc2;
+          float t2;
+          const float nu = fmaf(sy[j], d.y, base), nu_ = fmaf(-sy[j], d.y, base);
+          eval(nu, inc, t1);
+          eval(nu_, inc2, t2);
+          inc = fma3(inc2, make_float3(t2, t2, t2), inc * t1);
+          acc[j] = fma3(ground(nu_, ground(nu, inc)), cf, acc[j]);
+        }
+      }
+    }
+  }
+  if (GM == 1) {
+    const float4 g0 = gl[0], g1 = gl[1];
+#pragma unroll
+    for (int j = 0; j < kDensMaxGroup; ++j) {
+      if (j < G) {
+        const float w = (j == 0 && (ENDS || lo1)) || (j == jh && (ENDS || hi1)) ? 1.0f : 2.0f;
+        acc[j].x = fmaf(w, fmaf(g0.x, SC.x, g1.x * fmaf(sx[j], SX.x, mus_ct * SC.x)), acc[j].x);
+        acc[j].y = fmaf(w, fmaf(g0.y, SC.y, g1.y * fmaf(sx[j], SX.y, mus_ct * SC.y)), acc[j].y);
+        acc[j].z = fmaf(w, fmaf(g0.z, SC.z, g1.z * fmaf(sx[j], SX.z, mus_ct * SC.z)), acc[j].z);
       }
     }
   }
@@ -1084,6 +1213,7 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
     if (k < NT) {
       const ThetaRec t = thr[k];
       S.th[k] = t.th;
+      if (TWO) S.th[k].cos_t = fminf(fmaxf(t.th.cos_t, -1.0f), 1.0f);
       S.tay[k] = bounded_axis(t.tay, a.sc_mu);
     } else if (k < NT + ns) {
       const int c = k - NT, si = s0 + c;
@@ -1114,40 +1244,45 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
   // pre-scaled for line_pos
   const int MK = dens_mk(NNU, CL), MKE = dens_mke(a.ir_mus, CL);
   const int per_col = NT * MK;
-  LerpRec2* const P2 = reinterpret_cast<LerpRec2*>(S.P);  // order 2
+  // order 2: word w of record k of row l, column c
+  const int SL = dens2_slots(NNU);
+  auto P2 = [&](int c, int l, int w, int k) -> float4& { return S.P2[((c * NT + l) * 3 + w) * SL + k]; };
   const float hP = 0.5f * float(NNU - 1), hE = 0.5f * float(a.ir_mus - 1);
+  const float hD = TWO ? 1.0f : hP;  // scale of the direction table
   {
-    const float4* src0 = TWO ? a.dr : a.dms;
+    const float4* src0 = a.dms;
     // order 2: the Rayleigh and Mie tables carry their phase functions'
     // constants, 3 / (16 pi) and 3 / (8 pi) (1 - g^2) / (2 + g^2)
     const float sR = TWO ? 3.0f / (16.0f * kPiF) : 1.0f;
     const float sM = 3.0f / (8.0f * kPiF) * (1.0f - a.g * a.g) / (2.0f + a.g * a.g);
-    for (int k = tid; k < ns * per_col; k += nth) {
+    if (TWO) {
+      for (int e = tid; e < ns * NT * NNU; e += nth) {
+        const int c = e / (NT * NNU), l = (e / NNU) % NT, k = e % NNU;
+        const float3 v = fetch3(a.dr, a.W, a.sc_mu, S.kax[c * NK + k + 1], S.tay[l], s_az) * sR;
+        const float3 m = fetch3(a.dm, a.W, a.sc_mu, S.kax[c * NK + k + 1], S.tay[l], s_az) * sM;
+        P2(c, l, 0, k) = make_float4(v.x, v.y, v.z, 0.f);
+        P2(c, l, 1, k) = make_float4(0.f, 0.f, m.x, m.y);
+        P2(c, l, 2, k) = make_float4(m.z, 0.f, 0.f, 0.f);
+      }
+    }
+    for (int k = tid; !TWO && k < ns * per_col; k += nth) {
       const int c = k / per_col, l = (k % per_col) / MK, p = k % MK;
       // interval ki (-1 .. nu_size): left entry nu slice ki, kax index ki + 1
       const int ki = rec_interval<CL>(p, MK);
       const bool used = ki <= NNU;
       const int sl = ki + 1;
-      float3 v = make_float3(0.f, 0.f, 0.f), m = v;
-      if (used) {
-        v = fetch3(src0, a.W, a.sc_mu, S.kax[c * NK + sl], S.tay[l], s_az) * sR;
-        if (TWO) m = fetch3(a.dm, a.W, a.sc_mu, S.kax[c * NK + sl], S.tay[l], s_az) * sM;
-      }
-      if (!TWO) {
-        S.P[k].a = make_float4(v.x, v.y, v.z, 0.f);
-        S.P[k].b = S.P[k].pad = make_float2(0.f, 0.f);
-      } else {
-        P2[k].a = make_float4(v.x, v.y, v.z, 0.f);
-        P2[k].b = make_float4(0.f, 0.f, m.x, m.y);
-        P2[k].c = make_float4(m.z, 0.f, 0.f, 0.f);
-      }
+      float3 v = make_float3(0.f, 0.f, 0.f);
+      if (used)
+        v = fetch3(src0, a.W, a.sc_mu, S.kax[c * NK + sl], S.tay[l], s_az);
+      S.P[k].a = make_float4(v.x, v.y, v.z, 0.f);
+      S.P[k].b = S.P[k].pad = make_float2(0.f, 0.f);
     }
     const float dtheta = kPiF / float(NT), dphi = kPiF / float(NT);
     for (int k = tid; k < NT * NT; k += nth) {
       const int l = k / NT, m = k % NT;
       const float st = sinf((float(l) + 0.5f) * dtheta);
       const float phi = (float(m) + 0.5f) * dphi;
-      S.dir[k] = make_float2(cosf(phi) * st * hP, sinf(phi) * st * hP);
+      S.dir[k] = make_float2(cosf(phi) * st * hD, sinf(phi) * st * hD);
     }
     // ground rows: the ground table position we = A w + B0 + hE (r / R) mu_s
     for (int l = tid; l < NT; l += nth) {
@@ -1173,25 +1308,27 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
   }
   __syncthreads();
   {  // pass 2: differences of the two entries of each interval
-    for (int k = tid; k < ns * per_col; k += nth) {
+    for (int k = tid; !TWO && k < ns * per_col; k += nth) {
       const int p = k % MK, row0 = k - p, ki = rec_interval<CL>(p, MK);
       if (ki <= NNU - 1) {  // intervals -1 .. nu_size - 1
         const int right = row0 + rec_pos<CL>(ki + 1, MK);
-        if (!TWO) {
-          const float4 v0 = S.P[k].a, v1 = S.P[right].a;
-          S.P[k].b = make_float2(v1.x - v0.x, v1.y - v0.y);
-          S.P[k].pad = make_float2(v1.z - v0.z, 0.f);
-        } else {
-          // values only (the slope slots of `right` are being written by its owner)
-          LerpRec2& r0 = P2[k];
-          const LerpRec2& r1 = P2[right];
-          r0.a.w = r1.a.x - r0.a.x;
-          r0.b.x = r1.a.y - r0.a.y;
-          r0.b.y = r1.a.z - r0.a.z;
-          r0.c.y = r1.b.z - r0.b.z;
-          r0.c.z = r1.b.w - r0.b.w;
-          r0.c.w = r1.c.x - r0.c.x;
-        }
+        const float4 v0 = S.P[k].a, v1 = S.P[right].a;
+        S.P[k].b = make_float2(v1.x - v0.x, v1.y - v0.y);
+        S.P[k].pad = make_float2(v1.z - v0.z, 0.f);
+      }
+    }
+    if (TWO) {
+      for (int e = tid; e < ns * NT * (NNU - 1); e += nth) {
+        const int c = e / (NT * (NNU - 1)), l = (e / (NNU - 1)) % NT, k = e % (NNU - 1);
+        // values only (the slope fields of the next record are being written by its owner)
+        float4 &a0 = P2(c, l, 0, k), &b0 = P2(c, l, 1, k), &c0 = P2(c, l, 2, k);
+        const float4 &a1 = P2(c, l, 0, k + 1), &b1 = P2(c, l, 1, k + 1), &c1 = P2(c, l, 2, k + 1);
+        a0.w = a1.x - a0.x;
+        b0.x = a1.y - a0.y;
+        b0.y = a1.z - a0.z;
+        c0.y = b1.z - b0.z;
+        c0.z = b1.w - b0.w;
+        c0.w = c1.x - c0.x;
       }
     }
     for (int k = tid; k < MKE; k += nth) {  // intervals 0 .. ir_mus - 2 (-1 and ir_mus - 1: flat)
@@ -1204,38 +1341,58 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
     }
   }
   __syncthreads();
-  {  // pass 3: the line of interval ki, value at w = 0 and slope, in the record's own fields
+  {  // pass 3: the line of interval ki, value at w = 0 (order 2: nu = 0) and slope, in the record's own fields
     auto line = [](LerpRec& rec, int ki) {
       const float3 d = make_float3(rec.b.x, rec.b.y, rec.pad.x);
       const float c = 0.5f - float(ki);
       rec.a = make_float4(fmaf(c, d.x, rec.a.x), fmaf(c, d.y, rec.a.y), fmaf(c, d.z, rec.a.z), d.x);
       rec.b = make_float2(d.y, d.z);
     };
-    for (int k = tid; k < ns * per_col; k += nth) {
-      const int ki = rec_interval<CL>(k % MK, MK);
-      if (!TWO) {
-        line(S.P[k], ki);
-      } else {
-        LerpRec2& r = P2[k];
-        const float c = 0.5f - float(ki);
-        r.a.x = fmaf(c, r.a.w, r.a.x);
-        r.a.y = fmaf(c, r.b.x, r.a.y);
-        r.a.z = fmaf(c, r.b.y, r.a.z);
-        r.b.z = fmaf(c, r.c.y, r.b.z);
-        r.b.w = fmaf(c, r.c.z, r.b.w);
-        r.c.x = fmaf(c, r.c.w, r.c.x);
+    for (int k = tid; !TWO && k < ns * per_col; k += nth) line(S.P[k], rec_interval<CL>(k % MK, MK));
+    if (TWO) {
+      for (int e = tid; e < ns * NT * (NNU - 1); e += nth) {
+        const int cc = e / (NT * (NNU - 1)), l = (e / (NNU - 1)) % NT, k = e % (NNU - 1);
+        float4 &ra = P2(cc, l, 0, k), &rb = P2(cc, l, 1, k), &rc = P2(cc, l, 2, k);
+        const float c = hP - float(k);  // the table position of nu = 0 from entry k
+        ra = make_float4(fmaf(c, ra.w, ra.x), fmaf(c, rb.x, ra.y), fmaf(c, rb.y, ra.z), ra.w * hP);
+        rb = make_float4(rb.x * hP, rb.y * hP, fmaf(c, rc.y, rb.z), fmaf(c, rc.z, rb.w));
+        rc = make_float4(fmaf(c, rc.w, rc.x), rc.y * hP, rc.z * hP, rc.w * hP);
       }
     }
     for (int k = tid; k < MKE; k += nth) line(S.E[k], rec_interval<CL>(k, MKE));
   }
   __syncthreads();
+  if (TWO) {
+    // the kind of each theta row's ground bounce
+    for (int e = tid; e < ns * NT; e += nth) {
+      const int c = e / NT, l = e - c * NT;
+      const DensTheta t = S.th[l];
+      const float mus = S.col_mus[c], ss = sqrtf(gmax(a.g_cols[s0 + c].one_m_mus2, 0.0f));
+      const float2 g = S.gw[l];
+      const float gB = g.y + hE * (r / a.bottom) * mus;
+      const float w0 = fmaf(mus * hP, t.cos_t, hP - 0.5f), dw = hP * sinf((float(l) + 0.5f) * (kPiF / float(NT))) * ss;
+      const float we = fmaf(g.x, w0 - dw, gB), we1 = fmaf(g.x, w0 + dw, gB);
+      const int k = line_pos<CL>(we, MKE), k1 = line_pos<CL>(we1, MKE);
+      const LerpRec E = S.E[k];
+      // w = hP nu + hP - 1/2
+      const float gv = fmaf(g.x, hP - 0.5f, gB), gs = g.x * hP;
+      S.gl[2 * e] = make_float4(t.tgx * fmaf(E.a.w, gv, E.a.x), t.tgy * fmaf(E.b.x, gv, E.a.y),
+                                t.tgz * fmaf(E.b.y, gv, E.a.z), __int_as_float(!t.ground || k == k1 ? 1 : 2));
+      S.gl[2 * e + 1] = make_float4(t.tgx * E.a.w * gs, t.tgy * E.b.x * gs, t.tgz * E.b.y * gs, 0.f);
+    }
+    __syncthreads();
+  }
 
   // --- this thread's nu group
   const int per_s = sh.chunk * sh.NG;
-  const int cl = tid / per_s, yl = (tid % per_s) / sh.NG, grp = tid % sh.NG;
+  const int cl = tid / per_s, grp = (tid % per_s) / sh.chunk, yl = tid % sh.chunk;
   const bool active = tid < sh.S * per_s && cl < ns && yl < ny;
+  // order 2: whether the warp's first (last) texels are those at nu = -1 (1)
+  const bool lo1 = __all_sync(0xffffffffu, !active || grp == 0);
+  const bool hi1 = __all_sync(0xffffffffu, !active || grp == sh.NG - 1);
   if (active) {
     const int G = sh.G, y = y0 + yl, si = s0 + cl;
+    const int jh = NNU - 1 - (sh.NG - 1) * G;  // the texel at nu = 1 in the last group
     float mu = 0.f, ox = 0.f, mu_s;
     float sx[kDensMaxGroup], sy[kDensMaxGroup];
     // MIXED: the texel frame in FP64 (scattering.h:134-136 clamp, frame of
@@ -1260,7 +1417,7 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
     for (int j = 0; j < kDensMaxGroup; ++j) {
       sx[j] = sy[j] = 0.f;
       if (j < G) {
-        const int nu_i = grp * G + j, x = nu_i * a.sc_mus + si;
+        const int nu_i = min(grp * G + j, NNU - 1), x = nu_i * a.sc_mus + si;
         if (!MX) {
           mu = a.g_rows[zi * a.sc_mu + y].mu;
           const ColGeo& cg = a.g_cols[x];
@@ -1281,7 +1438,24 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
         }
       }
     }
+    if (TWO) {
+      // the two ends: the clamp leaves omega_s in the plane of omega (where
+      // omega is vertical, any plane: its phase functions do not depend on phi)
+      const float ss = sqrtf(gmax(a.g_cols[si].one_m_mus2, 0.0f));
+#pragma unroll
+      for (int j = 0; j < kDensMaxGroup; ++j) {
+        const bool lo = j == 0 && grp == 0, hi = j == jh && grp == sh.NG - 1;
+        if (lo || hi) {
+          sx[j] = lo ? -ss : ss;
+          sy[j] = 0.f;
+        }
+        // within [-1, 1], NaN included (fmaxf(NaN, -1) = -1)
+        sx[j] = fminf(fmaxf(sx[j], -1.0f), 1.0f);
+        sy[j] = fminf(fmaxf(sy[j], 0.0f), 1.0f);
+      }
+    }
     mu_s = S.col_mus[cl];
+    if (TWO) mu_s = fminf(fmaxf(mu_s, -1.0f), 1.0f);
     const float h0 = r - a.bottom;
     const float rho_r = profile_density(a.ray_d, h0), rho_m = profile_density(a.mie_d, h0);
     const float g = a.g;
@@ -1299,10 +1473,21 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
     q.oxs = ox / hP;
     q.offP = hP - 0.5f;
     q.gmus = hE * (r / a.bottom) * mu_s;
-    q.inv_h = 1.0f / hP;
-    q.c1 = 0.5f / hP - 1.0f;
     q.nP = MK;
     q.nE = MKE;
+    Dens2Const q2;
+    q2.mu = mu;
+    q2.mu_s = mu_s;
+    q2.ox = ox;
+    q2.scale = hP * kDens2Shrink;
+    q2.v_off = NNU & 1 ? 0.5f : 0.0f;
+    q2.g1 = pc.g1;
+    q2.g2 = pc.g2;
+    q2.gmus = q.gmus;
+    q2.hP = hP;
+    q2.k0 = (NNU - 1) / 2;
+    q2.slots = SL;
+    q2.nE = MKE;
     float3 acc[kDensMaxGroup];
 #pragma unroll
     for (int j = 0; j < kDensMaxGroup; ++j) acc[j] = make_float3(0.f, 0.f, 0.f);
@@ -1315,19 +1500,40 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
     }
     for (int l = 0; l < NT; ++l) {
       const DensTheta t = S.th[l];
-      const size_t row = (size_t)(cl * NT + l) * MK;
-      const LerpRec* Pl = TWO ? reinterpret_cast<const LerpRec*>(reinterpret_cast<const LerpRec2*>(S.P) + row)
-                              : S.P + row;
-      if (G == kDensMaxGroup) {
-        if (t.ground)
-          dens_row<TWO, true, CL, kDensMaxGroup>(S, t, l, NT, Pl, q, sx, sy, G, pc, acc);
-        else
-          dens_row<TWO, false, CL, kDensMaxGroup>(S, t, l, NT, Pl, q, sx, sy, G, pc, acc);
+      if (TWO) {
+        const float4* Pl = S.P2 + (size_t)(cl * NT + l) * 3 * SL;
+        const float4* gl = S.gl + 2 * (cl * NT + l);
+        const int kind = __float_as_int(gl[0].w);
+        auto rows = [&](auto gm) {
+          constexpr int GM = decltype(gm)::value;
+          if (NNU == 8)
+            dens_row2<GM, CL, 8, 8, true>(S, t, l, NT, Pl, gl, q2, sx, sy, G, jh, true, true, pc, acc);
+          else if (NNU == 4)
+            dens_row2<GM, CL, 4, 8, true>(S, t, l, NT, Pl, gl, q2, sx, sy, G, jh, true, true, pc, acc);
+          else if (NNU == 2)
+            dens_row2<GM, CL, 2, 8, true>(S, t, l, NT, Pl, gl, q2, sx, sy, G, jh, true, true, pc, acc);
+          else if (NNU < 8)
+            dens_row2<GM, CL, 0, 8, true>(S, t, l, NT, Pl, gl, q2, sx, sy, G, jh, true, true, pc, acc);
+          else if (NNU == 16)
+            dens_row2<GM, CL, 8, 16, false>(S, t, l, NT, Pl, gl, q2, sx, sy, G, jh, lo1, hi1, pc, acc);
+          else
+            dens_row2<GM, CL, 0, 0, false>(S, t, l, NT, Pl, gl, q2, sx, sy, G, jh, lo1, hi1, pc, acc);
+        };
+        if (kind == 1) rows(Int<1>());
+        else rows(Int<2>());
       } else {
-        if (t.ground)
-          dens_row<TWO, true, CL, 0>(S, t, l, NT, Pl, q, sx, sy, G, pc, acc);
-        else
-          dens_row<TWO, false, CL, 0>(S, t, l, NT, Pl, q, sx, sy, G, pc, acc);
+        const LerpRec* Pl = S.P + (size_t)(cl * NT + l) * MK;
+        if (G == kDensMaxGroup) {
+          if (t.ground)
+            dens_row<true, CL, kDensMaxGroup>(S, t, l, NT, Pl, q, sx, sy, G, pc, acc);
+          else
+            dens_row<false, CL, kDensMaxGroup>(S, t, l, NT, Pl, q, sx, sy, G, pc, acc);
+        } else {
+          if (t.ground)
+            dens_row<true, CL, 0>(S, t, l, NT, Pl, q, sx, sy, G, pc, acc);
+          else
+            dens_row<false, CL, 0>(S, t, l, NT, Pl, q, sx, sy, G, pc, acc);
+        }
       }
       if (MX && ((l + 1) % kDensKahanRows == 0 || l == NT - 1)) {
         // Kahan sum over theta rows of the FP32 sums over kDensKahanRows rows
@@ -1344,7 +1550,7 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
     }
 #pragma unroll
     for (int j = 0; j < kDensMaxGroup; ++j) {
-      if (j < G) {
+      if (j < G && grp * G + j < NNU) {
         const int x = (grp * G + j) * a.sc_mus + si;
         float* row = a.dens + ((size_t)zi * a.sc_mu + y) * 3 * a.Wd;
         float3 o = acc[j];
@@ -1352,6 +1558,8 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
           o = make_float3(accs[(6 * j) * kDensThreads] - accs[(6 * j + 3) * kDensThreads],
                           accs[(6 * j + 1) * kDensThreads] - accs[(6 * j + 4) * kDensThreads],
                           accs[(6 * j + 2) * kDensThreads] - accs[(6 * j + 5) * kDensThreads]);
+        // order 2: an end's sum holds one direction of each mirror pair
+        if (TWO && ((j == 0 && lo1) || (j == jh && hi1))) o = o * 2.0f;
         row[x] = store_round(o.x, a.f16);
         row[a.Wd + x] = store_round(o.y, a.f16);
         row[2 * a.Wd + x] = store_round(o.z, a.f16);
