@@ -643,24 +643,25 @@ void plan_group(Plan& P, const std::vector<DevAtmo>& A, const std::vector<int>& 
     D.variant = tuned % fb::kDensClamped + (cl ? fb::kDensClamped : 0);
     P.launches.push_back(D);
     }
-    PlannedLaunch M = mk(fb::kPassMultiple, n);
-    std::vector<int> tm;
-    for (int j : jobs) M.block = std::max(M.block, fb::ms_threads(A[j].W));
-    for (int j : jobs) {
-      const DevAtmo& a = A[j];
-      tm.push_back(fb::tiles_multiple(a.W, a.sc_mus, a.ms_steps, a.sc_mu, a.sc_r, M.block));
-      M.smem = std::max(M.smem, fb::ms_smem(a.W, a.ms_steps, a.sc_mus, M.block));
-      M.tpt = std::max(M.tpt, fb::ms_shape(a.W, a.sc_mus, a.ms_steps, M.block).TPT);
-      M.texels += (uint64_t)a.W * a.sc_mu * a.sc_r;
+    for (int v : {0, fb::kMsMid, fb::kMsWide, fb::kMsDefault, fb::kMsHalf, fb::kMsDouble}) {
+      std::vector<int> mj, tm;
+      for (int j : jobs)
+        if (fb::ms_variant(A[j].W, A[j].sc_mus) == v) mj.push_back(j);
+      if (mj.empty()) continue;
+      PlannedLaunch M = mk(fb::kPassMultiple, n);
+      M.block = fb::ms_layout(v).threads;
+      for (int j : mj) {
+        const DevAtmo& a = A[j];
+        tm.push_back(fb::tiles_multiple(a.W, a.sc_mus, a.ms_steps, a.sc_mu, a.sc_r, M.block));
+        M.smem = std::max(M.smem, fb::ms_smem(a.W, a.ms_steps, a.sc_mus, M.block));
+        M.tpt = std::max(M.tpt, fb::ms_shape(a.W, a.sc_mus, a.ms_steps, M.block).TPT);
+        M.texels += (uint64_t)a.W * a.sc_mu * a.sc_r;
+      }
+      add_segment(P, M, 0, mj, tm);
+      M.nseg = 1;
+      M.variant = v + (v == 0 || v == fb::kMsDefault ? launch_variant(A, mj, tun, mixed, false) : 0);
+      P.launches.push_back(M);
     }
-    add_segment(P, M, 0, jobs, tm);
-    M.nseg = 1;
-    M.variant = fb::ms_block_variant(M.block) >= 0 ? fb::ms_block_variant(M.block)
-                                                   : launch_variant(A, jobs, tun, mixed, false);
-    bool fixed = M.block == fb::kThreads && M.tpt == 1;
-    for (int j : jobs) fixed = fixed && fb::ms_fixed_layout(A[j].W, A[j].sc_mus);
-    if (fixed) M.variant += 4;  // 0, 1 -> 4, 5
-    P.launches.push_back(M);
   }
 }
 

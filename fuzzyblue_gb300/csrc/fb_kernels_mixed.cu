@@ -14,6 +14,8 @@ template __global__ void k_multiple<true, 1, 3>(LaunchArgs);
 template __global__ void k_multiple<true, 2, 3>(LaunchArgs);
 template __global__ void k_multiple<true, 1, 4>(LaunchArgs);
 template __global__ void k_multiple<true, 1, 5>(LaunchArgs);
+template __global__ void k_multiple<true, 1, 6>(LaunchArgs);
+template __global__ void k_multiple<true, 1, 7>(LaunchArgs);
 
 template __global__ void k_density_arcs<true, 2>(LaunchArgs);
 template __global__ void k_density_arcs<true, 6>(LaunchArgs);
@@ -59,6 +61,8 @@ const void* kernel_mixed(int pass, int tpt, int variant, bool order2) {
       if (variant == 3) return tpt >= 2 ? (const void*)k_multiple<true, 2, 3> : (const void*)k_multiple<true, 1, 3>;
       if (variant == 4 && tpt == 1) return (const void*)k_multiple<true, 1, 4>;
       if (variant == 5 && tpt == 1) return (const void*)k_multiple<true, 1, 5>;
+      if (variant == kMsHalf && tpt == 1) return (const void*)k_multiple<true, 1, kMsHalf>;
+      if (variant == kMsDouble && tpt == 1) return (const void*)k_multiple<true, 1, kMsDouble>;
       return v1 || variant == 5 ? (const void*)k_multiple<true, 1, 1> : (const void*)k_multiple<true, 1, 0>;
   }
   return nullptr;

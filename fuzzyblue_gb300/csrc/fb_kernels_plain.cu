@@ -15,6 +15,8 @@ template __global__ void k_multiple<false, 1, 3>(LaunchArgs);
 template __global__ void k_multiple<false, 2, 3>(LaunchArgs);
 template __global__ void k_multiple<false, 1, 4>(LaunchArgs);
 template __global__ void k_multiple<false, 1, 5>(LaunchArgs);
+template __global__ void k_multiple<false, 1, 6>(LaunchArgs);
+template __global__ void k_multiple<false, 1, 7>(LaunchArgs);
 
 template __global__ void k_density_arcs<false, 2>(LaunchArgs);
 template __global__ void k_density_arcs<false, 6>(LaunchArgs);
@@ -60,6 +62,8 @@ const void* kernel_plain(int pass, int tpt, int variant, bool order2) {
       if (variant == 3) return tpt >= 2 ? (const void*)k_multiple<false, 2, 3> : (const void*)k_multiple<false, 1, 3>;
       if (variant == 4 && tpt == 1) return (const void*)k_multiple<false, 1, 4>;
       if (variant == 5 && tpt == 1) return (const void*)k_multiple<false, 1, 5>;
+      if (variant == kMsHalf && tpt == 1) return (const void*)k_multiple<false, 1, kMsHalf>;
+      if (variant == kMsDouble && tpt == 1) return (const void*)k_multiple<false, 1, kMsDouble>;
       return v1 || variant == 5 ? (const void*)k_multiple<false, 1, 1> : (const void*)k_multiple<false, 1, 0>;
   }
   return nullptr;

@@ -14,8 +14,8 @@
 //   k_density_arcs     the same for orders >= 3              CTA per (r, mu_s columns, 32 mu rows)
 //                    indirect_irradiance.comp (segment 1)    CTA per irradiance r row (up to 64 texels);
 //                                                            order 1: four texels, a warp each
-//   k_multiple       multiple_scattering.comp                CTA per (mu, r) row(s); variants 4
-//                                                            and 5 compiled for the default layout
+//   k_multiple       multiple_scattering.comp                CTA per (mu, r) row(s); variants 4-7
+//                                                            compiled for the table classes' layouts
 // CTAs take work items from a global atomic counter; an item is a tile of one
 // atmosphere, located by binary search over per-atmosphere item offsets.
 #pragma once
@@ -1945,8 +1945,8 @@ namespace fb {
 // Tile of multiple scattering: whole rows (a texel's lookups can reach any
 // nu slice of its row: its clamped nu picks the slices), R = threads / W rows
 // per CTA for rows of at most `threads` texels, else one row with TPT texels
-// per thread. Launches use CTAs of kThreads threads; when a row of the launch
-// is wider, CTAs of kMsMidThreads (two per SM, so that one runs while the
+// per thread. Rows of up to kThreads texels have CTAs of that size; wider ones
+// CTAs of kMsMidThreads (two per SM, so that one runs while the
 // other waits at its per-sample barrier) up to rows of 512 texels, else of
 // kMsWideThreads (one texel per thread up to rows of 1024: measured faster
 // than two per thread on kMsMidThreads, which spill). The slab of a row holds,
@@ -1959,10 +1959,6 @@ constexpr int kMsMidThreads = 512;
 // are built.
 constexpr int kMsSlabs = 4;
 constexpr int kMsWideThreads = 1024;
-// The default table layout (32 mu_s texels, 8 nu slices), for which the
-// multiple-scattering kernels are also compiled with the sizes fixed (the
-// slab offsets of the texel loads become constants).
-constexpr int kMsFixedMuS = 32, kMsFixedW = 8 * kMsFixedMuS;
 constexpr int kMsRowBytes = 96 * 1024;  // shared memory for the rows of a tile (records + slabs)
 struct MSShape {
   int R;         // rows per tile
@@ -1977,19 +1973,28 @@ __host__ __device__ inline MSShape ms_shape(int W, int sc_mus, int steps, int th
   m.TPT = (m.R * W + threads - 1) / threads;
   return m;
 }
-// CTA size of a launch over rows of width W (the widest of the launch).
-__host__ __device__ inline int ms_threads(int W) {
-  return W <= kThreads ? kThreads : (W <= kMsMidThreads ? kMsMidThreads : kMsWideThreads);
+// Kernel variants: by CTA size, and for the layouts of the three table classes
+// compiled with their sizes, so that the slab offsets of the texel loads are
+// constants (mixed mode, order 2: 20 half-class atmospheres 0.285 -> 0.277 ms,
+// one of the double class 4.04 -> 3.89).
+constexpr int kMsMid = 3, kMsWide = 2, kMsDefault = 4, kMsHalf = 6, kMsDouble = 7;
+struct MSLayout {
+  int NM, W, threads;  // mu_s size and row width, 0 where not fixed; CTA size
+};
+__host__ __device__ constexpr MSLayout ms_layout(int variant) {
+  return variant == kMsWide     ? MSLayout{0, 0, kMsWideThreads}
+         : variant == kMsMid    ? MSLayout{0, 0, kMsMidThreads}
+         : variant == kMsHalf   ? MSLayout{16, 64, kThreads}
+         : variant == kMsDouble ? MSLayout{64, 1024, kMsWideThreads}
+         : variant >= kMsDefault ? MSLayout{32, 256, kThreads}  // 4, 5: the occupancy variants
+                                 : MSLayout{0, 0, kThreads};    // 0, 1
 }
-// Kernel variant of a launch of `block` threads: 2 and 3 for the wide CTA
-// sizes, -1 for kThreads (the tuned occupancy variant 0 or 1 applies).
-__host__ __device__ inline int ms_block_variant(int block) {
-  return block == kMsWideThreads ? 2 : (block == kMsMidThreads ? 3 : -1);
-}
-// An atmosphere of the fixed layout: with CTAs of kThreads (one texel per
-// thread) its launches may take variants 4 and 5.
-__host__ __device__ inline bool ms_fixed_layout(int W, int sc_mus) {
-  return W == kMsFixedW && sc_mus == kMsFixedMuS;
+// The variant of an atmosphere, before the tuned occupancy (+ 1 for variants 0
+// and 4). Each variant has a launch of its own: rows of one width fill its CTAs.
+__host__ __device__ inline int ms_variant(int W, int sc_mus) {
+  for (int v : {kMsDefault, kMsHalf, kMsDouble})
+    if (W == ms_layout(v).W && sc_mus == ms_layout(v).NM) return v;
+  return W <= kThreads ? 0 : (W <= kMsMidThreads ? kMsMid : kMsWide);
 }
 __host__ __device__ inline int tiles_multiple(int W, int sc_mus, int steps, int sc_mu, int sc_r, int threads) {
   const MSShape m = ms_shape(W, sc_mus, steps, threads);
@@ -2002,14 +2007,19 @@ __host__ __device__ inline size_t ms_smem(int W, int steps, int sc_mus, int thre
 
 // Position t in [0, n - 1] within a row of n texels as (i0, f): texel i0 in
 // [0, n - 1] and weight f of texel i0 + 1 (the value at t is p[i0] + f
-// (p[i0 + 1] - p[i0])); the clamp also maps NaN to 0. Rounding t - 1/2 to an
-// integer through the float adder gives floor(t), or floor(t) - 1 with f = 1
-// where t is an integer: the same interpolated value.
+// (p[i0 + 1] - p[i0])); the clamp also maps NaN to 0. The sum with 1.5 2^23
+// rounded down holds floor(t) in its low bits, returned with that constant's
+// bits on top.
 __device__ __forceinline__ int row_pos(float t, float n_minus_1, float& f) {
   t = fminf(fmaxf(t, 0.0f), n_minus_1);
-  const float y = (t - 0.5f) + kRoundMagic;
+  const float y = __fadd_rd(t, kRoundMagic);
   f = t - (y - kRoundMagic);
-  return max(__float_as_int(y) - kRoundMagicBits, 0);
+  return __float_as_int(y);
+}
+template <int OFF> __device__ __forceinline__ float ld_shared1(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1 + %2];" : "=f"(v) : "r"(addr), "n"(OFF));
+  return v;
 }
 
 // Compile-time switch of the multiple-scattering sample loop's lambdas.
@@ -2028,7 +2038,8 @@ __device__ void tile_multiple(const DevAtmo& a, int order, int tile, unsigned ch
   const int nrow = min(sh.R, nrows - row0);
   const int N = a.ms_steps, NS = N + 1;
   const int tid = threadIdx.x;
-  const int SR = sh.slab_row;                      // slab plane stride
+  constexpr int SRC = NMC ? (WC + NMC + 1 + 3) & ~3 : 0;
+  const int SR = SRC ? SRC : sh.slab_row;          // slab plane stride
   MSRec* rec = (MSRec*)smem;
   float* slab = (float*)(smem + align16(sizeof(MSRec) * (size_t)sh.R * NS));
   const int nx_tex = nrow * W;                     // texels of the tile = slab entries built per sample
@@ -2069,10 +2080,14 @@ __device__ void tile_multiple(const DevAtmo& a, int order, int tile, unsigned ch
   // are computed once, there, and copied. The tile's texels of the first and
   // last slices come first in the thread order, so that they share warps and
   // the other warps read one slice. Launch of order 2 over 16 default
-  // atmospheres, mixed: 3.70 -> 3.08 ms; the double class 4.66 -> 4.26 ms; the
-  // launch stays bound by the L1 data pipe (slab reads, density rows).
+  // atmospheres, mixed, 3.70 -> 3.08 ms; the slab units given to the warps of
+  // one slice, constant slab offsets and rows kept for every layout 2.89; the
+  // double class 4.66 -> 3.89, one default atmosphere in plain mode 0.293 ->
+  // 0.197. Bound by the L1 data pipe (84 % of its wavefronts: about a third
+  // density rows, a third slab reads).
   float c_rmus[TPT], c_nu[TPT], c_lerp[TPT];
   int c_lr[TPT], c_e[TPT], c_x[TPT], c_ro[TPT], c_from[TPT];
+  uint32_t c_addr[TPT];  // shared-memory address of the texel's slice in slab 0
   const int n_end = nrow * 2 * NM;  // texels of the first and last slices
   // per-unit constants of the slab build (TPT units per thread; a unit is
   // four entries of one plane of a row, and a tile has at most as many units
@@ -2090,7 +2105,9 @@ __device__ void tile_multiple(const DevAtmo& a, int order, int tile, unsigned ch
   bool all_full = true;
 #pragma unroll
   for (int j = 0; j < TPT; ++j) {
-    const int u0 = tid + j * nth, u = u0 < nunits ? u0 : u0 % nunits;
+    // from the last warp backwards: the first warps, whose texels take two
+    // slices, are those left without units
+    const int u0 = nth - 1 - tid + j * nth, u = u0 < nunits ? u0 : u0 % nunits;
     const int lr = u / (3 * G4), rem = u - lr * 3 * G4, pl = rem / G4, g = rem - pl * G4;
     u_ro[j] = lr * NS;
     u_src[j] = pl * a.Wd + 4 * g;
@@ -2149,6 +2166,10 @@ __device__ void tile_multiple(const DevAtmo& a, int order, int tile, unsigned ch
     } else {
       c_e[j] += slice * NM;
     }
+    // less the bits that row_pos leaves on top; through a shuffle, so that the
+    // assembler does not add these terms anew for each load
+    c_addr[j] = (uint32_t)__cvta_generic_to_shared(slab) + 4u * (uint32_t)(c_e[j] - kRoundMagicBits);
+    c_addr[j] = __shfl_sync(0xffffffffu, c_addr[j], tid & 31);
   }
   __syncthreads();
   const float* dens = a.dens;
@@ -2163,25 +2184,26 @@ __device__ void tile_multiple(const DevAtmo& a, int order, int tile, unsigned ch
   float4 q[TPT][4];
   // `fast` (MsFast<true>): the warp has a unit and a texel in every slot and
   // every unit is full, so the per-slot tests fold away
-  // Samples are loaded in order. With one row per tile (the fixed layout) all
-  // threads load the same four density rows, and a sample in the same (mu, r)
-  // cell as the one before (the offsets of two opposite corners fix all four)
-  // keeps the values already loaded.
+  // Samples are loaded in order: one in the same (mu, r) cell as the one before
+  // (the offsets of two opposite corners fix all four) keeps the values already
+  // loaded.
   int prev0 = -1, prev3 = -1;
   auto load = [&](auto fast, int i) {
 #pragma unroll
     for (int j = 0; j < TPT; ++j) {
       if (decltype(fast)::value || w_unit[j]) {
         const MSRec& o = rec[u_ro[j] + i];
-        if (NMC) {
-          const int o0 = o.off[0], o3 = o.off[3];
-          if (o0 == prev0 && o3 == prev3) continue;
-          prev0 = o0;
-          prev3 = o3;
+        const int4 off = *reinterpret_cast<const int4*>(o.off);
+        if (TPT == 1) {
+          if (off.x == prev0 && off.w == prev3) continue;
+          prev0 = off.x;
+          prev3 = off.w;
         }
         const float4* p = reinterpret_cast<const float4*>(dens + u_src[j]);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) q[j][c] = ld4(p + o.off[c]);
+        q[j][0] = ld4(p + off.x);
+        q[j][1] = ld4(p + off.y);
+        q[j][2] = ld4(p + off.z);
+        q[j][3] = ld4(p + off.w);
       }
     }
   };
@@ -2190,7 +2212,8 @@ __device__ void tile_multiple(const DevAtmo& a, int order, int tile, unsigned ch
     for (int j = 0; j < TPT; ++j) {
       if (decltype(fast)::value || w_unit[j]) {
         const MSRec& o = rec[u_ro[j] + i];
-        const float w00 = o.w[0], w10 = o.w[1], w01 = o.w[2], w11 = o.w[3];
+        const float4 w = *reinterpret_cast<const float4*>(o.w);
+        const float w00 = w.x, w10 = w.y, w01 = w.z, w11 = w.w;
         const float4 a00 = q[j][0], a10 = q[j][1], a01 = q[j][2], a11 = q[j][3];
         float4 v;
         v.x = fmaf(w11, a11.x, fmaf(w01, a01.x, fmaf(w10, a10.x, w00 * a00.x)));
@@ -2212,36 +2235,45 @@ __device__ void tile_multiple(const DevAtmo& a, int order, int tile, unsigned ch
   // the texel work of sample i on its slab; `close`: sample i ends a run of
   // the mixed sums (i % 8 == 7 or the last sample)
   // (`one`: every texel of the warp reads one slice)
-  auto step = [&](auto fast, auto one, int i, const float* cur, bool close) {
+  auto step = [&](auto fast, auto one, int i, uint32_t cur, bool close) {
 #pragma unroll
     for (int j = 0; j < TPT; ++j) {
       if (decltype(fast)::value || w_tex[j]) {
         const MSRec& o = rec[c_ro[j] + i];
+        const float4 o4 = *reinterpret_cast<const float4*>(&o);  // d, inv_r, tvwx, tvwy
         const float nu = c_nu[j];
         // position within a nu slice, texel units (scattering.h:48-56, 149-151):
         // both slices of the lookup share it
         float t;
         if (!MX) {
-          const float mu_s_i = clamp_cosine((c_rmus[j] + o.d * nu) * o.inv_r);
+          const float mu_s_i = fminf(fmaxf((c_rmus[j] + o4.x * nu) * o4.y, -1.0f), 1.0f);
           t = fmaf(musref.coord(mu_s_i), fmus, -0.5f);
         } else {
-          const float mu_s_i = clamp_cosine(fmaf(o.d, nu, c_rmus[j]) * o.inv_r);
+          const float mu_s_i = fminf(fmaxf(fmaf(o4.x, nu, c_rmus[j]) * o4.y, -1.0f), 1.0f);
           t = mus32.texel(mu_s_i);
         }
         float fx;
-        const int i0 = row_pos(t, fmus - 1.0f, fx);
-        const float* sl = cur + c_e[j] + i0;
-        const float* sg = sl + SR;
-        const float* sb = sl + 2 * SR;
-        float3 J = make_float3(fmaf(sl[1] - sl[0], fx, sl[0]), fmaf(sg[1] - sg[0], fx, sg[0]),
-                               fmaf(sb[1] - sb[0], fx, sb[0]));
+        const uint32_t at = ((uint32_t)row_pos(t, fmus - 1.0f, fx) << 2) + (c_addr[j] + cur);
+        // slab entries i0 and i0 + 1 of each plane, NM entries further on for
+        // the next slice; SRC: the plane stride where it is known
+        constexpr int P1 = 4 * SRC, P2 = 8 * SRC;
+        const uint32_t at1 = SRC ? at : at + 4 * SR, at2 = SRC ? at : at + 8 * SR;
+        const float r0 = ld_shared1<0>(at), r1 = ld_shared1<4>(at);
+        const float g0 = ld_shared1<P1>(at1), g1 = ld_shared1<P1 + 4>(at1);
+        const float b0 = ld_shared1<P2>(at2), b1 = ld_shared1<P2 + 4>(at2);
+        float3 J = make_float3(fmaf(r1 - r0, fx, r0), fmaf(g1 - g0, fx, g0), fmaf(b1 - b0, fx, b0));
         if (!decltype(one)::value && (decltype(fast)::value || w_two[j])) {
           const float lf = c_lerp[j];
-          const float bx = fmaf(sl[NM + 1] - sl[NM], fx, sl[NM]), by = fmaf(sg[NM + 1] - sg[NM], fx, sg[NM]);
-          const float bz = fmaf(sb[NM + 1] - sb[NM], fx, sb[NM]);
-          J = make_float3(fmaf(bx - J.x, lf, J.x), fmaf(by - J.y, lf, J.y), fmaf(bz - J.z, lf, J.z));
+          constexpr int N4 = 4 * NMC;
+          const uint32_t n4 = NMC ? 0u : 4u * (uint32_t)NM;
+          const float s0 = ld_shared1<N4>(at + n4), s1 = ld_shared1<N4 + 4>(at + n4);
+          const float h0 = ld_shared1<P1 + N4>(at1 + n4), h1 = ld_shared1<P1 + N4 + 4>(at1 + n4);
+          const float c0 = ld_shared1<P2 + N4>(at2 + n4), c1 = ld_shared1<P2 + N4 + 4>(at2 + n4);
+          J.x = fmaf(fmaf(s1 - s0, fx, s0) - J.x, lf, J.x);
+          J.y = fmaf(fmaf(h1 - h0, fx, h0) - J.y, lf, J.y);
+          J.z = fmaf(fmaf(c1 - c0, fx, c0) - J.z, lf, J.z);
         }
-        const float3 tvw = make_float3(o.tvwx, o.tvwy, o.tvwz);
+        const float3 tvw = make_float3(o4.z, o4.w, o.tvwz);
         if (!MX) {
           acc[j].s = fma3(J, tvw, acc[j].s);
         } else {
@@ -2255,99 +2287,78 @@ __device__ void tile_multiple(const DevAtmo& a, int order, int tile, unsigned ch
       }
     }
   };
-  // sample i lives in slab buffer i % kMsSlabs; with one texel per thread the
-  // loop runs four samples per iteration so that every buffer is a
-  // fixed pointer (with two, the longer body spills)
-  float* const sb0 = slab;
-  float* const sb1 = slab + slab_stride;
-  float* const sb2 = slab + 2 * slab_stride;
-  float* const sb3 = slab + 3 * slab_stride;
-  static_assert(kMsSlabs == 4, "four slab buffers");
-  // sample k from `cur` while sample k + A is built into `nxt`
+  // Two samples per barrier: i and i + 1 from their slabs, a pair of the four
+  // buffers, while i + 2 and i + 3 are built in the other pair.
+  static_assert(kMsSlabs == 4, "two pairs of slab buffers");
   const MsFast<false> slow;
   const MsFast<true> quick;
-  auto visit = [&](int k, const float* cur, float* nxt, int A) {
+  const uint32_t slab1 = WC && WC == NTH ? (uint32_t)(3 * SRC * 4) : (uint32_t)slab_stride * 4u;  // bytes from a slab to the next
+  const uint32_t pair = 2u * slab1;
+  float* const slab_b = slab;
+  auto buf = [&](uint32_t off) { return reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(slab_b) + off); };
+  auto visit = [&](int k, uint32_t cur, uint32_t nxt) {
     if (k < NS) {
-      if (kAhead && k + A < NS) load(slow, k + A);
+      if (kAhead && k + 2 < NS) load(slow, k + 2);
       step(slow, slow, k, cur, (k & 7) == 7 || k == N);
-      if (k + A < NS) {
-        if (!kAhead) load(slow, k + A);
-        blend(slow, k + A, nxt);
+      if (k + 2 < NS) {
+        if (!kAhead) load(slow, k + 2);
+        blend(slow, k + 2, buf(nxt));
       }
     }
   };
-  // the same where samples k and k + A exist; sample k ends a run if `close`
-  auto visit_full = [&](auto fast, auto one, int k, const float* cur, float* nxt, int A, bool close) {
-    if (kAhead) load(fast, k + A);
-    step(fast, one, k, cur, close);
-    if (!kAhead) load(fast, k + A);
-    blend(fast, k + A, nxt);
-  };
-  // warp-uniform: a unit and a texel in every slot, and those of one slice
-  const bool fast = TPT == 1 && all_full && w_unit[0] && w_tex[0], fast1 = fast && !w_two[0];
+  // What a warp does for a sample, decided once: 0 full units and texels of one
+  // slice, 1 full units and texels of two, 2 no units (texels of two slices), 3
+  // anything else
+  const int mode = TPT > 1 || !w_tex[0] ? 3 : (all_full && w_unit[0] ? (w_two[0] ? 1 : 0) : (w_unit[0] ? 3 : 2));
+  uint32_t cur = 0, nxt = pair;
   int i = 0;
-  // two samples per barrier: i and i + 1 from their slabs while i + 2 and
-  // i + 3 are built. The loops first take the samples whose successors two
-  // ahead exist, without bounds tests (plain mode, one default atmosphere, one
-  // sample per barrier with them: 0.285 ms, this way 0.279).
   load(slow, 0);
-  blend(slow, 0, sb0);
+  blend(slow, 0, buf(0));
   if (NS > 1) {
     load(slow, 1);
-    blend(slow, 1, sb1);
+    blend(slow, 1, buf(slab1));
   }
+  if (kAhead && mode < 2) load(quick, min(2, N));
   __syncthreads();
-  if (TPT == 1) {
-    for (; i + 5 < NS; i += 4) {
-      const bool c = (i & 4) != 0;  // sample i + 3 ends a run of 8
-      if (fast1) {
-        visit_full(quick, quick, i, sb0, sb2, 2, false);
-        visit_full(quick, quick, i + 1, sb1, sb3, 2, false);
-      } else if (fast) {
-        visit_full(quick, slow, i, sb0, sb2, 2, false);
-        visit_full(quick, slow, i + 1, sb1, sb3, 2, false);
-      } else {
-        visit_full(slow, slow, i, sb0, sb2, 2, false);
-        visit_full(slow, slow, i + 1, sb1, sb3, 2, false);
-      }
-      __syncthreads();
-      if (fast1) {
-        visit_full(quick, quick, i + 2, sb2, sb0, 2, false);
-        visit_full(quick, quick, i + 3, sb3, sb1, 2, c);
-      } else if (fast) {
-        visit_full(quick, slow, i + 2, sb2, sb0, 2, false);
-        visit_full(quick, slow, i + 3, sb3, sb1, 2, c);
-      } else {
-        visit_full(slow, slow, i + 2, sb2, sb0, 2, false);
-        visit_full(slow, slow, i + 3, sb3, sb1, 2, c);
-      }
-      __syncthreads();
+  // the samples whose successors two ahead exist, without bounds tests; the
+  // density rows of the next sample to build are requested before the barrier
+  for (; i + 3 < NS; i += 2) {
+    const bool c = (i & 7) == 6;  // sample i + 1 ends a run of 8
+    auto both = [&](auto one) {
+      step(quick, one, i, cur, false);
+      blend(quick, i + 2, buf(nxt));
+      load(quick, i + 3);
+      step(quick, one, i + 1, cur + slab1, c);
+      blend(quick, i + 3, buf(nxt + slab1));
+      load(quick, min(i + 4, N));
+    };
+    if (TPT == 1 && mode == 0) {
+      both(quick);
+    } else if (TPT == 1 && mode == 1) {
+      both(slow);
+    } else if (TPT == 1 && mode == 2) {
+      step(quick, slow, i, cur, false);
+      step(quick, slow, i + 1, cur + slab1, c);
+    } else {
+      if (kAhead) load(slow, i + 2);
+      step(slow, slow, i, cur, false);
+      if (!kAhead) load(slow, i + 2);
+      blend(slow, i + 2, buf(nxt));
+      if (kAhead) load(slow, i + 3);
+      step(slow, slow, i + 1, cur + slab1, c);
+      if (!kAhead) load(slow, i + 3);
+      blend(slow, i + 3, buf(nxt + slab1));
     }
-    for (; i < NS; i += 4) {
-      visit(i, sb0, sb2, 2);
-      visit(i + 1, sb1, sb3, 2);
-      __syncthreads();
-      visit(i + 2, sb2, sb0, 2);
-      visit(i + 3, sb3, sb1, 2);
-      __syncthreads();
-    }
-  } else {
-    for (; i + 3 < NS; i += 2) {
-      float* const b0 = slab + (i % kMsSlabs) * slab_stride;
-      float* const b1 = slab + ((i + 1) % kMsSlabs) * slab_stride;
-      float* const b2 = slab + ((i + 2) % kMsSlabs) * slab_stride;
-      float* const b3 = slab + ((i + 3) % kMsSlabs) * slab_stride;
-      // (a second copy for `fast` warps spills at this width)
-      const bool c = (i & 7) == 6;  // sample i + 1 ends a run of 8
-      visit_full(slow, slow, i, b0, b2, 2, false);
-      visit_full(slow, slow, i + 1, b1, b3, 2, c);
-      __syncthreads();
-    }
-    for (; i < NS; i += 2) {
-      visit(i, slab + (i % kMsSlabs) * slab_stride, slab + ((i + 2) % kMsSlabs) * slab_stride, 2);
-      visit(i + 1, slab + ((i + 1) % kMsSlabs) * slab_stride, slab + ((i + 3) % kMsSlabs) * slab_stride, 2);
-      __syncthreads();
-    }
+    __syncthreads();
+    cur ^= pair;
+    nxt ^= pair;
+  }
+  for (; i < NS; i += 2) {
+    visit(i, cur, nxt);
+    visit(i + 1, cur + slab1, nxt + slab1);
+    __syncthreads();
+    cur ^= pair;
+    nxt ^= pair;
   }
   // the ends' results to the texels that the clamp moves to them (the loops
   // end with a barrier: the slabs are no longer read)
@@ -2395,23 +2406,24 @@ __device__ void tile_multiple(const DevAtmo& a, int order, int tile, unsigned ch
 
 // V = 0: CTAs of kThreads, registers capped for 4 resident CTAs per SM;
 // V = 1: for 3; V = 2: CTAs of kMsWideThreads, one per SM; V = 3: CTAs of
-// kMsMidThreads, two per SM; V = 4, 5: as 0, 1 for launches whose atmospheres
-// all have the fixed layout (ms_fixed_layout), compiled with its sizes.
+// kMsMidThreads, two per SM; V = 4, 5: as 0, 1 for the default layout; V = 6, 7:
+// the half and the double class's layouts (ms_layout).
+constexpr int ms_ctas(int v) {
+  return ms_layout(v).threads == kMsWideThreads ? 1 : (v == kMsMid ? 2 : (v == 1 || v == kMsDefault + 1 ? 3 : 4));
+}
 template <bool MX, int TPT, int V>
-__global__ void __launch_bounds__(V == 2 ? kMsWideThreads : (V == 3 ? kMsMidThreads : kThreads),
-                                  V == 2 ? 1 : (V == 3 ? 2 : (V == 0 || V == 4 ? 4 : 3)))
-    k_multiple(LaunchArgs L) {
+__global__ void __launch_bounds__(ms_layout(V).threads, ms_ctas(V)) k_multiple(LaunchArgs L) {
   extern __shared__ __align__(16) unsigned char smem[];
   int seg, job, tile;
   int taken = 0;
-  constexpr int NTH = V == 2 ? kMsWideThreads : (V == 3 ? kMsMidThreads : kThreads);
-  constexpr bool FIX = V >= 4;
-  static_assert(!FIX || TPT == 1, "the fixed layout has one texel per thread");
+  constexpr MSLayout F = ms_layout(V);
+  constexpr int NTH = F.threads;
+  static_assert(!F.W || TPT == 1, "the fixed layouts have one texel per thread");
   if (blockDim.x != NTH) return;  // the launch plans give each variant its CTA size
   while (next_item(L, seg, job, tile, taken)) {
     const DevAtmo& a = L.atm[job];
-    if (FIX && !ms_fixed_layout(a.W, a.sc_mus)) continue;  // the launch plans never pair these
-    tile_multiple<MX, TPT, FIX ? kMsFixedMuS : 0, FIX ? kMsFixedW : 0, NTH>(a, L.order, tile, smem);
+    if (F.W && (a.W != F.W || a.sc_mus != F.NM)) continue;  // the launch plans never pair these
+    tile_multiple<MX, TPT, F.NM, F.W, NTH>(a, L.order, tile, smem);
   }
 }
 
