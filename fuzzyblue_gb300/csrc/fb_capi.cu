@@ -564,8 +564,8 @@ void plan_group(Plan& P, const std::vector<DevAtmo>& A, const std::vector<int>& 
           A[j].W, A[j].sc_mu, A[j].sc_r, mixed ? fb::irgeo_entries(A[j].ir_r, A[j].ir_mus, A[j].irr_n, A[j].sc_nu) : 0));
       L.texels += (uint64_t)A[j].tr_mu * A[j].tr_r;
     }
-    add_segment(P, L, 0, group, tiles);
-    add_segment(P, L, 1, group, tg);
+    add_segment(P, L, 0, group, tg);
+    add_segment(P, L, 1, group, tiles);
     L.nseg = 2;
     P.launches.push_back(L);
   }

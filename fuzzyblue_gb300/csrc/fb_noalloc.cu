@@ -236,8 +236,8 @@ extern "C" int fb_atmosphere_build_noalloc(void* stream, const fb_params* p, voi
   };
   const bool multi = d.order >= 2;
   rc = add(fb::kPassTransmittance, 0,
-           {fb::tiles_transmittance(d.tr_mu, d.tr_r),
-            fb::tiles_geometry(d.W, d.sc_mu, d.sc_r, mixed ? fb::irgeo_entries(d.ir_r, d.ir_mus, d.irr_n, d.sc_nu) : 0)},
+           {fb::tiles_geometry(d.W, d.sc_mu, d.sc_r, mixed ? fb::irgeo_entries(d.ir_r, d.ir_mus, d.irr_n, d.sc_nu) : 0),
+            fb::tiles_transmittance(d.tr_mu, d.tr_r)},
            0, 1, fb::kThreads, 0);
   if (!rc)
     rc = add(fb::kPassSingle, 0,
