@@ -28,16 +28,106 @@ __device__ __forceinline__ float3 f3add(float3 a, float3 b) { return make_float3
 __device__ __forceinline__ float f3dot(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ float f3len(float3 a) { return sqrtf(f3dot(a, a)); }
 
-// RGBA trilinear fetch (same weights and order as fetch3).
-__device__ float4 fetch3_rgba(const float4* t, int w, int h, Axis x, Axis y, Axis z) {
-  const float ia = 1.0f - x.f, ib = 1.0f - y.f, ic = 1.0f - z.f;
-  const float wt[8] = {ia * ib * ic, x.f * ib * ic, ia * y.f * ic, x.f * y.f * ic,
-                       ia * ib * z.f, x.f * ib * z.f, ia * y.f * z.f, x.f * y.f * z.f};
-  const int xs[2] = {x.i0, x.i1}, ys[2] = {y.i0, y.i1}, zs[2] = {z.i0, z.i1};
-  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+// What the sky pass needs of the atmosphere and the frame beside the tables: the
+// shaders' values that are the same for every pixel, each computed on the host by
+// the same FP32 operations, so that no pixel repeats their divisions and roots
+// (half of the pass's instructions). The camera's radius, sun cosine and lookup
+// axes among them, for a camera inside the atmosphere.
+struct SkyConst {
+  DevAtmo a;
+  DrawArgs d;
+  float H, RR, TT, HH;      // sqrt(T^2 - R^2), squares
+  // coord_from_unit(x, n) = c0 + x c1
+  float tr_mu0, tr_mu1, tr_r0, tr_r1, sc_r0, sc_r1, sc_mu0, sc_mu1, sc_mus0, sc_mus1;
+  float mus_dmin, mus_span, mus_A;  // u_mu_s: T - R, H - (T - R), A
+  float inv_nu;             // 1 / nu_size where that is exact (a power of two), else 0
+  float pr_k, pm_k, g1, g2; // phase functions
+  float mie_q;              // extrapolated Mie: rayleigh.x / mie_sca.x
+  float mie_c[3];           // mie_sca / rayleigh
+  float cam_r, cam_r2, cam_mu_s, mie_fade;  // |camera|, its square, sun cosine, smoothstep(0, 0.01, mu_s)
+};
+// A point's radius with the terms that the table coordinates share.
+struct PointTerms {
+  float r, rr, rho;
+  float u_r;        // scattering table
+  float v_tr;       // transmittance table
+  float d_min_t, span_t, d_min_g, span_g;  // T - r, rho + H - (T - r); r - R, rho - (r - R)
+  Axis az, atr;
+};
+__host__ __device__ inline Axis axis_of(float coord, int n) {
+  float x = coord * float(n) - 0.5f;
+  float fl = floorf(x);
+  Axis a;
+  a.f = x - fl;
+  fl = fminf(fmaxf(fl, -1.0f), float(n));
+  int i = (int)fl;
+  a.i0 = min(max(i, 0), n - 1);
+  a.i1 = min(max(i + 1, 0), n - 1);
+  return a;
+}
+__device__ __forceinline__ PointTerms point_terms(const SkyConst& k, float r) {
+  PointTerms p;
+  p.r = r;
+  p.rr = r * r;
+  p.rho = safe_sqrt(p.rr - k.RR);
+  const float x = p.rho / k.H;
+  p.u_r = k.sc_r0 + x * k.sc_r1;
+  p.v_tr = k.tr_r0 + x * k.tr_r1;
+  p.d_min_t = k.a.top - r;
+  p.span_t = (p.rho + k.H) - p.d_min_t;
+  p.d_min_g = r - k.a.bottom;
+  p.span_g = p.rho - p.d_min_g;
+  p.az = axis_of(p.u_r, k.a.sc_r);
+  p.atr = axis_of(p.v_tr, k.a.tr_r);
+  return p;
+}
+// transmittance.h:7-33
+__device__ __forceinline__ float3 sky_tr_to_top(const SkyConst& k, const PointTerms& p, float mu) {
+  const float disc = p.rr * (mu * mu - 1.0f) + k.TT;
+  const float d = gmax(-p.r * mu + safe_sqrt(disc), 0.0f);
+  const float x_mu = (d - p.d_min_t) / p.span_t;
+  return fetch2(k.a.tr, k.a.tr_mu, axis_of(k.tr_mu0 + x_mu * k.tr_mu1, k.a.tr_mu), p.atr);
+}
+// scattering.h:23-46
+__device__ __forceinline__ float sky_u_mu(const SkyConst& k, const PointTerms& p, float mu, bool ground) {
+  const float r_mu = p.r * mu;
+  const float disc = r_mu * r_mu - p.rr + k.RR;
+  if (ground) {
+    const float d = -r_mu - safe_sqrt(disc);
+    const float x = p.rho == p.d_min_g ? 0.0f : (d - p.d_min_g) / p.span_g;
+    return 0.5f - 0.5f * (k.sc_mu0 + x * k.sc_mu1);
+  }
+  const float d = -r_mu + safe_sqrt(disc + k.HH);
+  return 0.5f + 0.5f * (k.sc_mu0 + (d - p.d_min_t) / p.span_t * k.sc_mu1);
+}
+// scattering.h:48-56
+__host__ __device__ inline float sky_u_mu_s(const SkyConst& k, float mu_s) {
+  const float disc = k.RR * (mu_s * mu_s - 1.0f) + k.TT;
+  float d = -k.a.bottom * mu_s + sqrtf(disc < 0.0f ? 0.0f : disc);
+  d = d < 0.0f ? 0.0f : d;
+  const float aa = (d - k.mus_dmin) / k.mus_span;
+  float x = 1.0f - aa / k.mus_A;
+  x = x < 0.0f ? 0.0f : x;
+  return k.sc_mus0 + x / (1.0f + aa) * k.sc_mus1;
+}
+
+// render_sky.h:9-19
+__device__ __forceinline__ float3 extrapolated_single_mie(const SkyConst& k, float4 s) {
+  if (s.x <= 0.0f) return make_float3(0.f, 0.f, 0.f);
+  return make_float3(s.x * s.w / s.x * k.mie_q * k.mie_c[0], s.y * s.w / s.x * k.mie_q * k.mie_c[1],
+                     s.z * s.w / s.x * k.mie_q * k.mie_c[2]);
+}
+
+// RGBA trilinear fetch (same weights and order as fetch3) from the four rows that
+// both slices of a lookup share, row y of slice z in rows[2 z + y].
+__device__ __forceinline__ float4 fetch_rows(const float4* t, const uint32_t (&rows)[4], Axis x, float fy, float fz) {
+  const float ia = 1.0f - x.f, ib = 1.0f - fy, ic = 1.0f - fz;
+  const float wt[8] = {ia * ib * ic, x.f * ib * ic, ia * fy * ic, x.f * fy * ic,
+                       ia * ib * fz, x.f * ib * fz, ia * fy * fz, x.f * fy * fz};
+  float4 o;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    const float4 p = ld4(t + ((size_t)zs[k >> 2] * h + ys[(k >> 1) & 1]) * w + xs[k & 1]);
+    const float4 p = ld4(t + (rows[k >> 1] + (uint32_t)(k & 1 ? x.i1 : x.i0)));
     if (k == 0) {
       o = make_float4(wt[0] * p.x, wt[0] * p.y, wt[0] * p.z, wt[0] * p.w);
     } else {
@@ -50,97 +140,107 @@ __device__ float4 fetch3_rgba(const float4* t, int w, int h, Axis x, Axis y, Axi
   return o;
 }
 
-// render_sky.h:9-19
-__device__ float3 extrapolated_single_mie(const DevAtmo& a, float4 s) {
-  if (s.x <= 0.0f) return make_float3(0.f, 0.f, 0.f);
-  const float q = a.rayleigh[0] / a.mie_sca[0];
-  return make_float3(s.x * s.w / s.x * q * (a.mie_sca[0] / a.rayleigh[0]),
-                     s.y * s.w / s.x * q * (a.mie_sca[1] / a.rayleigh[1]),
-                     s.z * s.w / s.x * q * (a.mie_sca[2] / a.rayleigh[2]));
-}
-
-// render_sky.h:21-43 (scattering.h:7-60 for the coordinates)
-__device__ float3 combined_scattering(const DevAtmo& a, const Geo32& G, float r, float mu, float mu_s, float nu,
-                                      bool ground, float3& single_mie) {
-  const float u_r = G.u_r(a, r), u_mu = G.u_mu(a, r, mu, ground), u_mu_s = G.u_mu_s(a, mu_s);
-  const float u_nu = (nu + 1.0f) / 2.0f;
-  const float tcx = u_nu * float(a.sc_nu - 1);
-  const float tex_x = floorf(tcx);
-  const float lerp = tcx - tex_x;
-  const Axis ay = make_axis(u_mu, a.sc_mu), az = make_axis(u_r, a.sc_r);
-  const float4 s0 = fetch3_rgba(a.sc, a.W, a.sc_mu, make_axis((tex_x + u_mu_s) / float(a.sc_nu), a.W), ay, az);
-  const float4 s1 =
-      fetch3_rgba(a.sc, a.W, a.sc_mu, make_axis((tex_x + 1.0f + u_mu_s) / float(a.sc_nu), a.W), ay, az);
+// render_sky.h:21-43 (scattering.h:7-60 for the coordinates): tex_x and lerp are
+// the lookup's nu slice and weight
+__device__ __forceinline__ float3 combined_scattering(const SkyConst& k, const PointTerms& p, float mu, float u_mu_s,
+                                                      float tex_x, float lerp, bool ground, float3& single_mie) {
+  const DevAtmo& a = k.a;
+  const Axis ay = axis_of(sky_u_mu(k, p, mu, ground), a.sc_mu);
+  // (the table has at most 2^30 texels)
+  const uint32_t z0 = (uint32_t)(p.az.i0 * a.sc_mu), z1 = (uint32_t)(p.az.i1 * a.sc_mu), W = (uint32_t)a.W;
+  const uint32_t rows[4] = {(z0 + ay.i0) * W, (z0 + ay.i1) * W, (z1 + ay.i0) * W, (z1 + ay.i1) * W};
+  const float x0 = tex_x + u_mu_s, x1 = tex_x + 1.0f + u_mu_s;
+  float u0, u1;
+  if (k.inv_nu != 0.0f) {
+    u0 = x0 * k.inv_nu;
+    u1 = x1 * k.inv_nu;
+  } else {
+    u0 = x0 / float(a.sc_nu);
+    u1 = x1 / float(a.sc_nu);
+  }
+  const float4 s0 = fetch_rows(a.sc, rows, axis_of(u0, a.W), ay.f, p.az.f);
+  const float4 s1 = fetch_rows(a.sc, rows, axis_of(u1, a.W), ay.f, p.az.f);
   const float il = 1.0f - lerp;
   const float4 m = make_float4(s0.x * il + s1.x * lerp, s0.y * il + s1.y * lerp, s0.z * il + s1.z * lerp,
                                s0.w * il + s1.w * lerp);
-  single_mie = extrapolated_single_mie(a, m);
+  single_mie = extrapolated_single_mie(k, m);
   return make_float3(m.x, m.y, m.z);
 }
 
 // render_sky.h:111-191 without light shafts (shadow_length 0)
-__device__ float3 sky_radiance_to_point(const DevAtmo& a, const Geo32& G, float3 camera, float3 view, float3 point,
-                                        float3 sun, float3& transmittance) {
-  float r = f3len(camera);
+__device__ __forceinline__ float3 sky_radiance_to_point(const SkyConst& k, float3 view, float3 point, float3& transmittance) {
+  const DevAtmo& a = k.a;
+  float3 camera = make_float3(k.d.cam[0], k.d.cam[1], k.d.cam[2]);
+  const float3 sun = make_float3(k.d.sun[0], k.d.sun[1], k.d.sun[2]);
+  float r = k.cam_r, mu_s = k.cam_mu_s;
   float rmu = f3dot(camera, view);
-  const float to_top = -rmu - sqrtf(rmu * rmu - r * r + a.top * a.top);
+  const float to_top = -rmu - sqrtf(rmu * rmu - k.cam_r2 + k.TT);
   if (to_top > 0.0f) {
     camera = f3add(camera, view * to_top);
     r = a.top;
     rmu += to_top;
+    mu_s = f3dot(camera, sun) / r;
   } else if (r > a.top) {
     transmittance = make_float3(1.f, 1.f, 1.f);
     return make_float3(0.f, 0.f, 0.f);
   }
+  const PointTerms pc = point_terms(k, r);
   const float mu = rmu / r;
-  const float mu_s = f3dot(camera, sun) / r;
   const float nu = f3dot(view, sun);
   const float d = f3len(f3sub(point, camera));
-  const bool ground = G.hits_ground(r, mu);
-  transmittance = G.tr_segment(a, r, mu, d, ground);
+  const bool ground = mu < 0.0f && pc.rr * (mu * mu - 1.0f) + k.RR >= 0.0f;
+  // transmittance.h:35-61; the point's radius serves the scattering lookup too
+  const float r_p = gclamp(sqrtf(d * d + 2.0f * r * mu * d + pc.rr), a.bottom, a.top);
+  const float mu_p = (r * mu + d) / r_p;
+  const PointTerms pp = point_terms(k, r_p);
+  {
+    const float mu_d = clamp_cosine(mu_p);
+    const float3 tc = sky_tr_to_top(k, pc, ground ? -mu : mu), td = sky_tr_to_top(k, pp, ground ? -mu_d : mu_d);
+    transmittance = min1(ground ? td / tc : tc / td);
+  }
+  const float tcx = (nu + 1.0f) / 2.0f * float(a.sc_nu - 1);
+  const float tex_x = floorf(tcx), lerp = tcx - tex_x;
   float3 single_mie;
-  float3 scattering = combined_scattering(a, G, r, mu, mu_s, nu, ground, single_mie);
+  float3 scattering = combined_scattering(k, pc, mu, sky_u_mu_s(k, mu_s), tex_x, lerp, ground, single_mie);
   if (!isinf(d)) {
-    const float r_p = G.clamp_radius(sqrtf(d * d + 2.0f * r * mu * d + r * r));
-    const float mu_p = (r * mu + d) / r_p;
     const float mu_s_p = (r * mu_s + d * nu) / r_p;
     float3 single_mie_p;
-    const float3 scattering_p = combined_scattering(a, G, r_p, mu_p, mu_s_p, nu, ground, single_mie_p);
+    const float3 scattering_p = combined_scattering(k, pp, mu_p, sky_u_mu_s(k, mu_s_p), tex_x, lerp, ground, single_mie_p);
     const float3 shadow = transmittance;
     scattering = f3sub(scattering, shadow * scattering_p);
     single_mie = f3sub(single_mie, shadow * single_mie_p);
-    single_mie = extrapolated_single_mie(a, make_float4(scattering.x, scattering.y, scattering.z, single_mie.x));
-    single_mie = single_mie * smoothstepf(0.0f, 0.01f, mu_s);
+    single_mie = extrapolated_single_mie(k, make_float4(scattering.x, scattering.y, scattering.z, single_mie.x));
+    single_mie = single_mie * (mu_s == k.cam_mu_s ? k.mie_fade : smoothstepf(0.0f, 0.01f, mu_s));
   }
-  const float pr = phase_rayleigh(nu), pm = phase_mie(a.g, nu);
+  // util.h:26-34
+  const float gg = k.g1 - k.g2 * nu;  // to the power 3/2 as a product with its root
+  const float pr = k.pr_k * (1.0f + nu * nu), pm = k.pm_k * (1.0f + nu * nu) / (gg * sqrtf(gg));
   return f3add(scattering * pr, single_mie * pm);
 }
 
-__global__ void __launch_bounds__(256) k_render_sky(DevAtmo a, DrawArgs d, const float* depth, uint32_t width,
-                                                    uint32_t height, float4* color, float4* trans) {
-  const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= (uint64_t)width * height) return;
-  const uint32_t x = (uint32_t)(k % width), y = (uint32_t)(k / width);
-  Geo32 G;
-  G.init(a);
+__global__ void __launch_bounds__(256) k_render_sky(const __grid_constant__ SkyConst k, const float* depth,
+                                                    uint32_t width, uint32_t height, float4* color, float4* trans) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (uint64_t)width * height) return;
+  const uint32_t n = (uint32_t)i;  // at most 2^31 pixels
+  const uint32_t y = n / width, x = n - y * width;
   // render_sky.frag:24-34
   const float sx = 2.0f * ((float(x) + 0.5f) / float(width)) - 1.0f;
   const float sy = 2.0f * ((float(y) + 0.5f) / float(height)) - 1.0f;
-  const float dz = depth ? depth[k] : 0.0f;
+  const float dz = depth ? depth[n] : 0.0f;
   float v[4], w[4];
 #pragma unroll
   for (int row = 0; row < 4; ++row) {
-    v[row] = d.m[0][row] * sx + d.m[1][row] * sy + d.m[2][row] * 0.0f + d.m[3][row] * 1.0f;
-    w[row] = d.m[0][row] * sx + d.m[1][row] * sy + d.m[2][row] * dz + d.m[3][row] * 1.0f;
+    v[row] = k.d.m[0][row] * sx + k.d.m[1][row] * sy + k.d.m[2][row] * 0.0f + k.d.m[3][row] * 1.0f;
+    w[row] = k.d.m[0][row] * sx + k.d.m[1][row] * sy + k.d.m[2][row] * dz + k.d.m[3][row] * 1.0f;
   }
   const float vl = f3len(make_float3(v[0], v[1], v[2]));
   const float3 view = make_float3(v[0] / vl, v[1] / vl, v[2] / vl);
   const float3 world = make_float3(w[0] / w[3] * 1e-3f, w[1] / w[3] * 1e-3f, w[2] / w[3] * 1e-3f);
   float3 t;
-  const float3 c = sky_radiance_to_point(a, G, make_float3(d.cam[0], d.cam[1], d.cam[2]), view, world,
-                                         make_float3(d.sun[0], d.sun[1], d.sun[2]), t);
-  color[k] = make_float4(c.x, c.y, c.z, 0.0f);
-  if (trans) trans[k] = make_float4(t.x, t.y, t.z, 1.0f);
+  const float3 c = sky_radiance_to_point(k, view, world, t);
+  color[n] = make_float4(c.x, c.y, c.z, 0.0f);
+  if (trans) trans[n] = make_float4(t.x, t.y, t.z, 1.0f);
 }
 
 // render_lighting.h:10-28 (irradiance.h:20-38, transmittance.h:63-74)
@@ -180,6 +280,43 @@ int record_of(const fb_atmosphere* atm, DevAtmo& d) {
   return FB_OK;
 }
 
+// The per-frame values, by the shaders' FP32 operations (this unit's host code is
+// compiled without contraction too).
+void fill_sky_const(SkyConst& k) {
+  const DevAtmo& a = k.a;
+  const float R = a.bottom, T = a.top;
+  k.RR = R * R;
+  k.TT = T * T;
+  k.H = sqrtf(k.TT - k.RR);
+  k.HH = k.H * k.H;
+  auto unit = [](int n, float& c0, float& c1) {
+    c0 = 0.5f / float(n);
+    c1 = 1.0f - 1.0f / float(n);
+  };
+  unit(a.tr_mu, k.tr_mu0, k.tr_mu1);
+  unit(a.tr_r, k.tr_r0, k.tr_r1);
+  unit(a.sc_r, k.sc_r0, k.sc_r1);
+  unit(a.sc_mu / 2, k.sc_mu0, k.sc_mu1);
+  unit(a.sc_mus, k.sc_mus0, k.sc_mus1);
+  k.mus_dmin = T - R;
+  k.mus_span = k.H - k.mus_dmin;
+  k.mus_A = -2.0f * a.mu_s_min * R / k.mus_span;
+  k.inv_nu = (a.sc_nu & (a.sc_nu - 1)) == 0 ? 1.0f / float(a.sc_nu) : 0.0f;
+  k.pr_k = 3.0f / (16.0f * kPiF);
+  k.pm_k = 3.0f / (8.0f * kPiF) * (1.0f - a.g * a.g) / (2.0f + a.g * a.g);
+  k.g1 = 1.0f + a.g * a.g;
+  k.g2 = 2.0f * a.g;
+  k.mie_q = a.rayleigh[0] / a.mie_sca[0];
+  for (int c = 0; c < 3; ++c) k.mie_c[c] = a.mie_sca[c] / a.rayleigh[c];
+  const float* cam = k.d.cam;
+  k.cam_r = sqrtf(cam[0] * cam[0] + cam[1] * cam[1] + cam[2] * cam[2]);
+  k.cam_r2 = k.cam_r * k.cam_r;
+  k.cam_mu_s = (cam[0] * k.d.sun[0] + cam[1] * k.d.sun[1] + cam[2] * k.d.sun[2]) / k.cam_r;
+  float t = (k.cam_mu_s - 0.0f) / (0.01f - 0.0f);
+  t = t < 0.0f ? 0.0f : (1.0f < t ? 1.0f : t);
+  k.mie_fade = t * t * (3.0f - 2.0f * t);
+}
+
 }  // namespace
 
 extern "C" int fb_atmosphere_render_sky(const fb_atmosphere* a, void* stream, const fb_draw_parameters* dp,
@@ -190,18 +327,18 @@ extern "C" int fb_atmosphere_render_sky(const fb_atmosphere* a, void* stream, co
     return fbi::set_error(FB_ERR_INVALID_ARGUMENT, "image size out of range");
   if (((uintptr_t)color | (uintptr_t)transmittance) & 15u)
     return fbi::set_error(FB_ERR_INVALID_ARGUMENT, "output images must be 16-byte aligned");
-  DevAtmo d;
-  record_of(a, d);
-  DrawArgs args;
+  SkyConst k;
+  record_of(a, k.a);
   for (int c = 0; c < 4; ++c)
-    for (int r = 0; r < 4; ++r) args.m[c][r] = dp->inverse_viewproj[c][r];
+    for (int r = 0; r < 4; ++r) k.d.m[c][r] = dp->inverse_viewproj[c][r];
   for (int i = 0; i < 3; ++i) {
-    args.cam[i] = dp->camera_position[i];
-    args.sun[i] = dp->sun_direction[i];
+    k.d.cam[i] = dp->camera_position[i];
+    k.d.sun[i] = dp->sun_direction[i];
   }
+  fill_sky_const(k);
   const uint64_t n = (uint64_t)width * height;
-  k_render_sky<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(d, args, depth, width, height,
-                                                                             (float4*)color, (float4*)transmittance);
+  k_render_sky<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(k, depth, width, height, (float4*)color,
+                                                                             (float4*)transmittance);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fbi::set_error(FB_ERR_CUDA, cudaGetErrorString(e));
   return FB_OK;
