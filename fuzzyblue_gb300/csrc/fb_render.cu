@@ -28,11 +28,21 @@ __device__ __forceinline__ float3 f3add(float3 a, float3 b) { return make_float3
 __device__ __forceinline__ float f3dot(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ float f3len(float3 a) { return sqrtf(f3dot(a, a)); }
 
+// A point's radius with the terms that the table coordinates share.
+struct PointTerms {
+  float r, rr, rho;
+  float u_r;        // scattering table
+  float v_tr;       // transmittance table
+  float d_min_t, span_t, d_min_g, span_g;  // T - r, rho + H - (T - r); r - R, rho - (r - R)
+  Axis az, atr;
+};
 // What the sky pass needs of the atmosphere and the frame beside the tables: the
 // shaders' values that are the same for every pixel, each computed on the host by
-// the same FP32 operations, so that no pixel repeats their divisions and roots
-// (half of the pass's instructions). The camera's radius, sun cosine and lookup
-// axes among them, for a camera inside the atmosphere.
+// the same FP32 operations, so that no pixel repeats their divisions and roots:
+// the camera's radius, sun cosine and lookup axes among them, for a camera inside
+// the atmosphere. A frame of 1920 x 1080 with depth 146 -> 96 us, bound by issue
+// (some 1450 instructions per pixel, of them 22 correctly rounded divisions, which
+// the differences of nearly equal lookups need).
 struct SkyConst {
   DevAtmo a;
   DrawArgs d;
@@ -45,31 +55,25 @@ struct SkyConst {
   float mie_q;              // extrapolated Mie: rayleigh.x / mie_sca.x
   float mie_c[3];           // mie_sca / rayleigh
   float cam_r, cam_r2, cam_mu_s, mie_fade;  // |camera|, its square, sun cosine, smoothstep(0, 0.01, mu_s)
-};
-// A point's radius with the terms that the table coordinates share.
-struct PointTerms {
-  float r, rr, rho;
-  float u_r;        // scattering table
-  float v_tr;       // transmittance table
-  float d_min_t, span_t, d_min_g, span_g;  // T - r, rho + H - (T - r); r - R, rho - (r - R)
-  Axis az, atr;
+  float cam_u_mu_s;
+  PointTerms cam;
 };
 __host__ __device__ inline Axis axis_of(float coord, int n) {
   float x = coord * float(n) - 0.5f;
   float fl = floorf(x);
   Axis a;
-  a.f = x - fl;
-  fl = fminf(fmaxf(fl, -1.0f), float(n));
+  a.f = x - fl;  // (NaN where x is infinite or NaN; the indices stay in range whatever the conversion gives)
   int i = (int)fl;
   a.i0 = min(max(i, 0), n - 1);
   a.i1 = min(max(i + 1, 0), n - 1);
   return a;
 }
-__device__ __forceinline__ PointTerms point_terms(const SkyConst& k, float r) {
+__host__ __device__ inline PointTerms point_terms(const SkyConst& k, float r) {
   PointTerms p;
   p.r = r;
   p.rr = r * r;
-  p.rho = safe_sqrt(p.rr - k.RR);
+  const float q = p.rr - k.RR;
+  p.rho = sqrtf(q < 0.0f ? 0.0f : q);
   const float x = p.rho / k.H;
   p.u_r = k.sc_r0 + x * k.sc_r1;
   p.v_tr = k.tr_r0 + x * k.tr_r1;
@@ -111,14 +115,19 @@ __host__ __device__ inline float sky_u_mu_s(const SkyConst& k, float mu_s) {
   return k.sc_mus0 + x / (1.0f + aa) * k.sc_mus1;
 }
 
-// render_sky.h:9-19
+// render_sky.h:9-19: the red channel, and all three with the hardware quotient
+// (the result only scales the image; the red one goes into a difference)
+__device__ __forceinline__ float extrapolated_mie_red(const SkyConst& k, float4 s) {
+  return s.x <= 0.0f ? 0.0f : s.x * s.w / s.x * k.mie_q * k.mie_c[0];
+}
 __device__ __forceinline__ float3 extrapolated_single_mie(const SkyConst& k, float4 s) {
   if (s.x <= 0.0f) return make_float3(0.f, 0.f, 0.f);
-  return make_float3(s.x * s.w / s.x * k.mie_q * k.mie_c[0], s.y * s.w / s.x * k.mie_q * k.mie_c[1],
-                     s.z * s.w / s.x * k.mie_q * k.mie_c[2]);
+  const float q = __fdividef(s.w, s.x) * k.mie_q;
+  return make_float3(s.x * q * k.mie_c[0], s.y * q * k.mie_c[1], s.z * q * k.mie_c[2]);
 }
 
-// RGBA trilinear fetch (same weights and order as fetch3) from the four rows that
+// RGBA trilinear fetch (weights, order and rounding of fetch3: near points show
+// the difference of two lookups that agree in most digits) from the four rows that
 // both slices of a lookup share, row y of slice z in rows[2 z + y].
 __device__ __forceinline__ float4 fetch_rows(const float4* t, const uint32_t (&rows)[4], Axis x, float fy, float fz) {
   const float ia = 1.0f - x.f, ib = 1.0f - fy, ic = 1.0f - fz;
@@ -142,8 +151,8 @@ __device__ __forceinline__ float4 fetch_rows(const float4* t, const uint32_t (&r
 
 // render_sky.h:21-43 (scattering.h:7-60 for the coordinates): tex_x and lerp are
 // the lookup's nu slice and weight
-__device__ __forceinline__ float3 combined_scattering(const SkyConst& k, const PointTerms& p, float mu, float u_mu_s,
-                                                      float tex_x, float lerp, bool ground, float3& single_mie) {
+__device__ __forceinline__ float4 combined_scattering(const SkyConst& k, const PointTerms& p, float mu, float u_mu_s,
+                                                      float tex_x, float lerp, bool ground) {
   const DevAtmo& a = k.a;
   const Axis ay = axis_of(sky_u_mu(k, p, mu, ground), a.sc_mu);
   // (the table has at most 2^30 texels)
@@ -161,10 +170,8 @@ __device__ __forceinline__ float3 combined_scattering(const SkyConst& k, const P
   const float4 s0 = fetch_rows(a.sc, rows, axis_of(u0, a.W), ay.f, p.az.f);
   const float4 s1 = fetch_rows(a.sc, rows, axis_of(u1, a.W), ay.f, p.az.f);
   const float il = 1.0f - lerp;
-  const float4 m = make_float4(s0.x * il + s1.x * lerp, s0.y * il + s1.y * lerp, s0.z * il + s1.z * lerp,
-                               s0.w * il + s1.w * lerp);
-  single_mie = extrapolated_single_mie(k, m);
-  return make_float3(m.x, m.y, m.z);
+  return make_float4(s0.x * il + s1.x * lerp, s0.y * il + s1.y * lerp, s0.z * il + s1.z * lerp,
+                     s0.w * il + s1.w * lerp);
 }
 
 // render_sky.h:111-191 without light shafts (shadow_length 0)
@@ -172,7 +179,8 @@ __device__ __forceinline__ float3 sky_radiance_to_point(const SkyConst& k, float
   const DevAtmo& a = k.a;
   float3 camera = make_float3(k.d.cam[0], k.d.cam[1], k.d.cam[2]);
   const float3 sun = make_float3(k.d.sun[0], k.d.sun[1], k.d.sun[2]);
-  float r = k.cam_r, mu_s = k.cam_mu_s;
+  float r = k.cam_r, mu_s = k.cam_mu_s, u_mu_s = k.cam_u_mu_s, fade = k.mie_fade;
+  PointTerms pc = k.cam;
   float rmu = f3dot(camera, view);
   const float to_top = -rmu - sqrtf(rmu * rmu - k.cam_r2 + k.TT);
   if (to_top > 0.0f) {
@@ -180,11 +188,13 @@ __device__ __forceinline__ float3 sky_radiance_to_point(const SkyConst& k, float
     r = a.top;
     rmu += to_top;
     mu_s = f3dot(camera, sun) / r;
+    u_mu_s = sky_u_mu_s(k, mu_s);
+    fade = smoothstepf(0.0f, 0.01f, mu_s);
+    pc = point_terms(k, r);
   } else if (r > a.top) {
     transmittance = make_float3(1.f, 1.f, 1.f);
     return make_float3(0.f, 0.f, 0.f);
   }
-  const PointTerms pc = point_terms(k, r);
   const float mu = rmu / r;
   const float nu = f3dot(view, sun);
   const float d = f3len(f3sub(point, camera));
@@ -200,21 +210,21 @@ __device__ __forceinline__ float3 sky_radiance_to_point(const SkyConst& k, float
   }
   const float tcx = (nu + 1.0f) / 2.0f * float(a.sc_nu - 1);
   const float tex_x = floorf(tcx), lerp = tcx - tex_x;
-  float3 single_mie;
-  float3 scattering = combined_scattering(k, pc, mu, sky_u_mu_s(k, mu_s), tex_x, lerp, ground, single_mie);
+  const float4 m = combined_scattering(k, pc, mu, u_mu_s, tex_x, lerp, ground);
+  float3 scattering = make_float3(m.x, m.y, m.z), single_mie;
   if (!isinf(d)) {
     const float mu_s_p = (r * mu_s + d * nu) / r_p;
-    float3 single_mie_p;
-    const float3 scattering_p = combined_scattering(k, pp, mu_p, sky_u_mu_s(k, mu_s_p), tex_x, lerp, ground, single_mie_p);
+    const float4 mp = combined_scattering(k, pp, mu_p, sky_u_mu_s(k, mu_s_p), tex_x, lerp, ground);
     const float3 shadow = transmittance;
-    scattering = f3sub(scattering, shadow * scattering_p);
-    single_mie = f3sub(single_mie, shadow * single_mie_p);
-    single_mie = extrapolated_single_mie(k, make_float4(scattering.x, scattering.y, scattering.z, single_mie.x));
-    single_mie = single_mie * (mu_s == k.cam_mu_s ? k.mie_fade : smoothstepf(0.0f, 0.01f, mu_s));
+    scattering = f3sub(scattering, shadow * make_float3(mp.x, mp.y, mp.z));
+    const float red = extrapolated_mie_red(k, m) - shadow.x * extrapolated_mie_red(k, mp);
+    single_mie = extrapolated_single_mie(k, make_float4(scattering.x, scattering.y, scattering.z, red)) * fade;
+  } else {
+    single_mie = extrapolated_single_mie(k, m);
   }
   // util.h:26-34
-  const float gg = k.g1 - k.g2 * nu;  // to the power 3/2 as a product with its root
-  const float pr = k.pr_k * (1.0f + nu * nu), pm = k.pm_k * (1.0f + nu * nu) / (gg * sqrtf(gg));
+  const float gs = rsqrtf(k.g1 - k.g2 * nu);
+  const float pr = k.pr_k * (1.0f + nu * nu), pm = k.pm_k * (1.0f + nu * nu) * (gs * gs * gs);
   return f3add(scattering * pr, single_mie * pm);
 }
 
@@ -315,6 +325,8 @@ void fill_sky_const(SkyConst& k) {
   float t = (k.cam_mu_s - 0.0f) / (0.01f - 0.0f);
   t = t < 0.0f ? 0.0f : (1.0f < t ? 1.0f : t);
   k.mie_fade = t * t * (3.0f - 2.0f * t);
+  k.cam_u_mu_s = sky_u_mu_s(k, k.cam_mu_s);
+  k.cam = point_terms(k, k.cam_r);
 }
 
 }  // namespace
