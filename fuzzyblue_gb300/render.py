@@ -66,20 +66,33 @@ class DrawParameters:
                               sun_direction=tuple(float(x) for x in sun))
 
 
+_Float3 = ctypes.c_float * 3
+
+
+def _stream(stream) -> Optional[int]:
+    """The handle of `stream`, or of the current stream of the current device:
+    asked for as such, a torch.cuda.Stream object costs 3 us to build, as much as
+    the launch."""
+    if stream is None:
+        import torch
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    from .api import _stream_handle
+    return _stream_handle(stream)
+
+
 def render_sky(atmosphere, draw: DrawParameters, width: int, height: int, depth=None, stream=None):
     """The sky pass for a width x height image: returns (radiance, transmittance)
     as torch tensors of shape (height, width, 4) on the atmosphere's device.
     `depth`: an optional (height, width) float32 CUDA tensor."""
     import torch
-    from .api import _stream_handle
     color = torch.empty((height, width, 4), dtype=torch.float32, device="cuda")
-    trans = torch.empty((height, width, 4), dtype=torch.float32, device="cuda")
+    trans = torch.empty_like(color)
     dptr = None
     if depth is not None:
         assert depth.is_cuda and depth.dtype == torch.float32 and tuple(depth.shape) == (height, width)
         dptr = depth.contiguous().data_ptr()
     c = draw.to_c()
-    s = _stream_handle(stream) if stream is not None else torch.cuda.current_stream().cuda_stream
+    s = _stream(stream)
     N.check(N.lib().fb_atmosphere_render_sky(atmosphere._h, s, ctypes.byref(c), dptr, width, height,
                                              color.data_ptr(), trans.data_ptr()), "fb_atmosphere_render_sky")
     return color, trans
@@ -89,14 +102,13 @@ def sun_and_sky_irradiance(atmosphere, points, normals, sun_direction, stream=No
     """GetSunAndSkyIrradiance at points (n, 3) with normals (n, 3), km, as
     CUDA tensors: returns (sun irradiance, sky irradiance), each (n, 3)."""
     import torch
-    from .api import _stream_handle
     points = points.contiguous().float()
     normals = normals.contiguous().float()
     n = int(points.shape[0])
     sun_out = torch.empty((n, 3), dtype=torch.float32, device="cuda")
-    sky_out = torch.empty((n, 3), dtype=torch.float32, device="cuda")
-    sd = (ctypes.c_float * 3)(*[float(x) for x in sun_direction])
-    s = _stream_handle(stream) if stream is not None else torch.cuda.current_stream().cuda_stream
+    sky_out = torch.empty_like(sun_out)
+    sd = _Float3(*[float(x) for x in sun_direction])
+    s = _stream(stream)
     N.check(N.lib().fb_atmosphere_sun_and_sky_irradiance(atmosphere._h, s, points.data_ptr(), normals.data_ptr(),
                                                          sd, n, sun_out.data_ptr(), sky_out.data_ptr()),
             "fb_atmosphere_sun_and_sky_irradiance")
