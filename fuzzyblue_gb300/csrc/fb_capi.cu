@@ -581,7 +581,7 @@ void plan_group(Plan& P, const std::vector<DevAtmo>& A, const std::vector<int>& 
         t2.push_back(fb::tiles_msrec(a.sc_mu, a.sc_r, a.ms_steps));
         t3.push_back(fb::tiles_densgeo(a.sc_r, a.dens_n));
       }
-      L.smem = std::max(L.smem, fb::ss_smem(a.W, a.ss_steps, a.sc_mus, a.sc_nu));
+      L.smem = std::max(L.smem, fb::ss_smem(a.W, a.ss_steps, a.sc_mu * a.sc_r));
       L.texels += (uint64_t)a.W * a.sc_mu * a.sc_r + (uint64_t)a.ir_mus * a.ir_r;
     }
     add_segment(P, L, 0, group, t0);
@@ -653,8 +653,8 @@ void plan_group(Plan& P, const std::vector<DevAtmo>& A, const std::vector<int>& 
       for (int j : mj) {
         const DevAtmo& a = A[j];
         tm.push_back(fb::tiles_multiple(a.W, a.sc_mus, a.ms_steps, a.sc_mu, a.sc_r, M.block));
-        M.smem = std::max(M.smem, fb::ms_smem(a.W, a.ms_steps, a.sc_mus, M.block));
-        M.tpt = std::max(M.tpt, fb::ms_shape(a.W, a.sc_mus, a.ms_steps, M.block).TPT);
+        M.smem = std::max(M.smem, fb::ms_smem(a.W, a.ms_steps, a.sc_mus, a.sc_mu * a.sc_r, M.block));
+        M.tpt = std::max(M.tpt, fb::ms_shape(a.W, a.sc_mus, a.ms_steps, a.sc_mu * a.sc_r, M.block).TPT);
         M.texels += (uint64_t)a.W * a.sc_mu * a.sc_r;
       }
       add_segment(P, M, 0, mj, tm);

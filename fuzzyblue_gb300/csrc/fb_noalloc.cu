@@ -243,9 +243,9 @@ extern "C" int fb_atmosphere_build_noalloc(void* stream, const fb_params* p, voi
     rc = add(fb::kPassSingle, 0,
              {fb::tiles_rows(d.W, d.sc_mu, d.sc_r), fb::tiles_direct(d.ir_mus, d.ir_r),
               multi ? fb::tiles_msrec(d.sc_mu, d.sc_r, d.ms_steps) : 0, multi ? fb::tiles_densgeo(d.sc_r, d.dens_n) : 0},
-             fb::ss_smem(d.W, d.ss_steps, d.sc_mus, d.sc_nu), 1, fb::kThreads, 0);
+             fb::ss_smem(d.W, d.ss_steps, d.sc_mu * d.sc_r), 1, fb::kThreads, 0);
   const int ms_variant = fb::ms_variant(d.W, d.sc_mus), ms_block = fb::ms_layout(ms_variant).threads;
-  const int ms_tpt = fb::ms_shape(d.W, d.sc_mus, d.ms_steps, ms_block).TPT;
+  const int ms_tpt = fb::ms_shape(d.W, d.sc_mus, d.ms_steps, d.sc_mu * d.sc_r, ms_block).TPT;
   for (int n = 2; !rc && n <= d.order; ++n) {
     if (n >= 3 && d.arcs) {
       const fb::ArcShape sh = fb::arc_shape(d.sc_r, d.sc_mu, d.sc_mus, d.sc_nu);
@@ -262,7 +262,7 @@ extern "C" int fb_atmosphere_build_noalloc(void* stream, const fb_params* p, voi
     }
     if (!rc)
       rc = add(fb::kPassMultiple, n, {fb::tiles_multiple(d.W, d.sc_mus, d.ms_steps, d.sc_mu, d.sc_r, ms_block)},
-               fb::ms_smem(d.W, d.ms_steps, d.sc_mus, ms_block), ms_tpt, ms_block, ms_variant);
+               fb::ms_smem(d.W, d.ms_steps, d.sc_mus, d.sc_mu * d.sc_r, ms_block), ms_tpt, ms_block, ms_variant);
   }
   if (rc) return rc;
 

@@ -55,7 +55,10 @@ struct LaunchArgs {
 };
 
 // Takes the next work item of the launch for this CTA; `taken` counts the
-// items this CTA has taken (for LaunchArgs::max_items).
+// items this CTA has taken (for LaunchArgs::max_items). (Asking for an item
+// while the one before is worked on hides the counter's round trip but commits
+// CTAs to items that others would be free for: the order-2 density of one
+// default atmosphere went from 0.61 to 0.63 ms, of odd sizes from 0.29 to 0.54.)
 __device__ __forceinline__ bool next_item(const LaunchArgs& L, int& seg, int& job, int& tile, int& taken) {
   __shared__ int s_item;
   if (L.max_items > 0 && taken >= L.max_items) return false;
@@ -477,7 +480,24 @@ __device__ __forceinline__ void texel_mus_nu(const RowGeo& ri, const ColGeo& c, 
   r_mu_s = ri.r * mu_s;
 }
 
-__host__ __device__ inline int rows_per_tile(int W) { return W >= kThreads ? 1 : kThreads / W; }
+// Tables of fewer tiles than the GPU has SMs split a tile's serial work among its
+// threads (single and multiple scattering the samples, density the theta rows).
+constexpr int kFillTiles = 152;
+// Single scattering: rows per tile, and the threads that share a texel's samples
+// (smoke sizes, 16 tiles: 40 -> 15 us).
+struct SSShape {
+  int R, SG;
+};
+__host__ __device__ inline SSShape ss_shape(int W, int rows) {
+  SSShape s;
+  s.R = W >= kThreads ? 1 : kThreads / W;
+  s.SG = 1;
+  while (s.SG < 8 && s.R >= 2 && rows < kFillTiles * s.R) {
+    s.SG *= 2;
+    s.R /= 2;
+  }
+  return s;
+}
 
 // ======================================================= MS sample records ===
 // multiple_scattering.comp:19-40, the parts that depend on the view ray and
@@ -659,10 +679,11 @@ struct __align__(16) SSRec {
 };
 
 
-template <bool MX>
+template <bool MX, bool SPLIT>
 __device__ void tile_single(const DevAtmo& a, int tile, unsigned char* smem) {
   const int W = a.W, nrows = a.sc_mu * a.sc_r;
-  const int R = rows_per_tile(W);
+  const SSShape sh = ss_shape(W, nrows);
+  const int R = sh.R, SG = SPLIT ? sh.SG : 1;
   const int row0 = tile * R;
   const int nrow = min(R, nrows - row0);
   const int N = a.ss_steps, NS = N + 1;
@@ -757,7 +778,12 @@ __device__ void tile_single(const DevAtmo& a, int tile, unsigned char* smem) {
   // transmittance lookups) lie closer together than those of a warp along
   // mu_s, so its lookups touch fewer cache sectors.
   const int NU = a.sc_nu, NMS = a.sc_mus;
-  for (int k = tid; k < nrow * W; k += kThreads) {
+  // With SG > 1 the tile has a texel for each run of SG threads at most, and
+  // thread group g takes a share of its samples.
+  const int ntex = nrow * W, nper = (NS + SG - 1) / SG;
+  for (int k2 = tid; k2 < ntex || (SPLIT && k2 < kThreads); k2 += kThreads) {
+    const int g = SPLIT ? k2 / ntex : 0, k = k2 - g * ntex;
+    const int i_end = !SPLIT ? NS : (g < SG ? min(NS, (g + 1) * nper) : 0);
     const int lr = k / W, kx = k - lr * W, kn = kx / NU;
     const int x = (kx - kn * NU) * NMS + kn;  // nu slice kx % NU, mu_s column kx / NU
     const RowGeo& ri = rows[lr];
@@ -767,7 +793,7 @@ __device__ void tile_single(const DevAtmo& a, int tile, unsigned char* smem) {
     Kahan3 ray, mie;
     ray.init();
     mie.init();
-    for (int i = 0; i < NS; ++i) {
+    for (int i = SPLIT ? g * nper : 0; i < i_end; ++i) {
       const SSRec& o = rr[i];
       float x_mu, mu_s_d;
       if (!MX) {
@@ -810,8 +836,22 @@ __device__ void tile_single(const DevAtmo& a, int tile, unsigned char* smem) {
       }
     }
     const float dx = MX ? (float)(ri.distd / double(N)) : ri.dist / float(N);
-    const float3 rs = MX ? make_float3(ray.s.x - ray.c.x, ray.s.y - ray.c.y, ray.s.z - ray.c.z) : ray.s;
-    const float3 ms = MX ? make_float3(mie.s.x - mie.c.x, mie.s.y - mie.c.y, mie.s.z - mie.c.z) : mie.s;
+    float3 rs = MX ? make_float3(ray.s.x - ray.c.x, ray.s.y - ray.c.y, ray.s.z - ray.c.z) : ray.s;
+    float3 ms = MX ? make_float3(mie.s.x - mie.c.x, mie.s.y - mie.c.y, mie.s.z - mie.c.z) : mie.s;
+    if (SPLIT) {  // (one pass of the loop, all threads)
+      float* x = reinterpret_cast<float*>(rec);
+      __syncthreads();  // the records are no longer read
+      const float v[6] = {rs.x, rs.y, rs.z, ms.x, ms.y, ms.z};
+#pragma unroll
+      for (int q = 0; q < 6; ++q) x[q * kThreads + tid] = v[q];
+      __syncthreads();
+      if (g > 0) break;
+      for (int h = 1; h < SG; ++h) {
+        const float* o = x + h * ntex + k;
+        rs = rs + make_float3(o[0], o[kThreads], o[2 * kThreads]);
+        ms = ms + make_float3(o[3 * kThreads], o[4 * kThreads], o[5 * kThreads]);
+      }
+    }
     const float3 R3 = rs * dx * ld3(a.solar) * ld3(a.rayleigh);
     const float3 M3 = ms * dx * ld3(a.solar) * ld3(a.mie_sca);
     const size_t t = (size_t)(row0 + lr) * W + x;
@@ -833,7 +873,11 @@ template <bool MX> __global__ void __launch_bounds__(kThreads, 4) k_single(Launc
   int seg, job, tile;
   int taken = 0;
   while (next_item(L, seg, job, tile, taken)) {
-    if (seg == 0) tile_single<MX>(L.atm[job], tile, smem);
+    if (seg == 0) {
+      const DevAtmo& a = L.atm[job];
+      if (ss_shape(a.W, a.sc_mu * a.sc_r).SG > 1) tile_single<MX, true>(a, tile, smem);
+      else tile_single<MX, false>(a, tile, smem);
+    }
     else if (seg == 1) tile_direct<MX>(L.atm[job], tile);
     else if (seg == 2) tile_msrec<MX>(L.atm[job], tile);
     else tile_densgeo<MX>(L.atm[job], tile);
@@ -857,12 +901,19 @@ template <bool MX> __global__ void __launch_bounds__(kThreads, 4) k_single(Launc
 constexpr int kDensThreads = 128;
 constexpr int kDensMaxGroup = 8;
 
+// Tables of fewer density tiles split a texel's theta rows among up to four threads
+// (smoke sizes, 16 tiles: 47 -> 27 us). The line lies below the half class's 128
+// tiles: one atmosphere of it would gain (117 -> 86 us), a batch of 20 lose (0.767
+// -> 0.841 ms), as every tile reads the tables of all theta rows.
+constexpr int kDensFillTiles = 100;
+
 // Per-atmosphere tile shape of the density pass (host and device agree).
 struct DensShape {
   int G;      // texels per thread (<= kDensMaxGroup; the last group of a row may have fewer)
   int NG;     // nu groups per mu row
   int S;      // mu_s columns per tile
   int chunk;  // mu rows per tile
+  int LS;     // thread groups that share a texel's theta rows
   int scols, ychunks, tiles;
 };
 // S_req / chunk_req: a tile shape chosen by the autotuner (0 = default rule:
@@ -873,14 +924,18 @@ __host__ __device__ inline DensShape dens_shape(int sc_r, int sc_mu, int sc_mus,
   d.NG = (sc_nu + kDensMaxGroup - 1) / kDensMaxGroup;
   d.G = (sc_nu + d.NG - 1) / d.NG;
   const int per_col = sc_mu * d.NG;
-  if (S_req > 0 && chunk_req > 0 && S_req * min(chunk_req, sc_mu) * d.NG <= kDensThreads) {
+  // (by the table's sizes alone: a tuned shape changes no sum)
+  d.LS = 1;
+  while (d.LS < 4 && per_col * sc_mus * sc_r * d.LS < kDensFillTiles * kDensThreads && d.NG * 2 * d.LS <= kDensThreads) d.LS *= 2;
+  const int threads = kDensThreads / d.LS;
+  if (S_req > 0 && chunk_req > 0 && S_req * min(chunk_req, sc_mu) * d.NG <= threads) {
     d.S = min(S_req, sc_mus);
     d.chunk = min(chunk_req, sc_mu);
-  } else if (per_col >= kDensThreads) {
+  } else if (per_col >= threads) {
     d.S = 1;
-    d.chunk = max(1, kDensThreads / d.NG);
+    d.chunk = max(1, threads / d.NG);
   } else {
-    d.S = max(1, min(sc_mus, kDensThreads / per_col));
+    d.S = max(1, min(sc_mus, threads / per_col));
     d.chunk = sc_mu;
   }
   // the interval tables grow with S (nu + 2) records per theta row: with many
@@ -960,11 +1015,11 @@ struct DensLayout {
   double* col_musd; // S (MIXED)
   double2* ymu;     // chunk (MIXED): (mu, 1 - mu^2)
   double* nuraw;    // sc_nu (MIXED)
-  float* acc;       // kDensThreads * kDensMaxGroup * 3 * 2 (MIXED: Kahan sum over theta rows)
+  float* acc;       // kDensThreads * kDensMaxGroup * 3 * 2 (MIXED: Kahan sum over theta rows) or 3 (PLAIN: LS > 1)
 };
 
 __host__ __device__ inline size_t dens_layout(unsigned char* base, int dens_n, int sc_nu, int ir_mus, int S,
-                                              int chunk, bool two, bool mixed, bool cl, DensLayout* L) {
+                                              int chunk, bool two, bool mixed, bool cl, int LS, DensLayout* L) {
   const int NT = dens_n, NK = sc_nu + 2;
   const size_t p_bytes = two ? sizeof(float4) * S * NT * 3 * dens2_slots(sc_nu)
                              : sizeof(LerpRec) * S * NT * dens_mk(sc_nu, cl);
@@ -979,7 +1034,7 @@ __host__ __device__ inline size_t dens_layout(unsigned char* base, int dens_n, i
   size_t o_P = take(p_bytes), o_gl = take(two ? sizeof(float4) * S * NT * 2 : 0), o_E = take(sizeof(LerpRec) * dens_mke(ir_mus, cl));
   size_t o_cm = take(sizeof(float) * S), o_cmd = take(sizeof(double) * S);
   size_t o_ymu = take(mixed ? sizeof(double2) * chunk : 0), o_nu = take(mixed ? sizeof(double) * sc_nu : 0);
-  size_t o_acc = take(mixed ? sizeof(float) * kDensThreads * kDensMaxGroup * 6 : 0);
+  size_t o_acc = take(sizeof(float) * kDensThreads * kDensMaxGroup * (mixed ? 6 : LS > 1 ? 3 : 0));
   if (L) {
     L->th = (DensTheta*)(base + o_th);
     L->tay = (Axis*)(base + o_tay);
@@ -1259,7 +1314,7 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
   const int ns = min(sh.S, a.sc_mus - s0), ny = min(sh.chunk, a.sc_mu - y0);
   const int tid = threadIdx.x, nth = blockDim.x;
   DensLayout S;
-  dens_layout(smem, NT, NNU, a.ir_mus, sh.S, sh.chunk, TWO, MX, CL, &S);
+  dens_layout(smem, NT, NNU, a.ir_mus, sh.S, sh.chunk, TWO, MX, CL, sh.LS, &S);
 
   // --- tile scalars (r slice), theta rows, columns and mu rows from the
   // geometry tables
@@ -1443,14 +1498,28 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
 
   // --- this thread's nu group
   const int per_s = sh.chunk * sh.NG;
-  const int cl = tid / per_s, grp = (tid % per_s) / sh.chunk, yl = tid % sh.chunk;
-  const bool active = tid < sh.S * per_s && cl < ns && yl < ny;
+  // ls: the share of the theta rows (LS of them, each of whole warps)
+  const int cap = kDensThreads / sh.LS, ls = tid / cap, gt = tid - ls * cap;
+  const int cl = gt / per_s, grp = (gt % per_s) / sh.chunk, yl = gt % sh.chunk;
+  const bool active = gt < sh.S * per_s && cl < ns && yl < ny;
   // order 2: whether the warp's first (last) texels are those at nu = -1 (1)
   const bool lo1 = __all_sync(0xffffffffu, !active || grp == 0);
   const bool hi1 = __all_sync(0xffffffffu, !active || grp == sh.NG - 1);
+  const int nq = (NT + sh.LS - 1) / sh.LS, l_end = min(NT, (ls + 1) * nq);
+  const int G = sh.G, y = y0 + yl, si = s0 + cl;
+  const int jh = NNU - 1 - (sh.NG - 1) * G;  // the texel at nu = 1 in the last group
+  // (sum, compensation) x 3 x G per thread, element e at accs[e * kDensThreads]:
+  // consecutive threads use consecutive banks, offsets are immediates
+  volatile float* accs = S.acc + tid;
+  // texel j's density; order 2: an end's sum holds one direction of each mirror pair
+  auto store = [&](int j, float3 o) {
+    if (TWO && ((j == 0 && lo1) || (j == jh && hi1))) o = o * 2.0f;
+    float* row = a.dens + ((size_t)zi * a.sc_mu + y) * 3 * a.Wd + (grp * G + j) * a.sc_mus + si;
+    row[0] = store_round(o.x, a.f16);
+    row[a.Wd] = store_round(o.y, a.f16);
+    row[2 * a.Wd] = store_round(o.z, a.f16);
+  };
   if (active) {
-    const int G = sh.G, y = y0 + yl, si = s0 + cl;
-    const int jh = NNU - 1 - (sh.NG - 1) * G;  // the texel at nu = 1 in the last group
     float mu = 0.f, ox = 0.f, mu_s;
     float sx[kDensMaxGroup], sy[kDensMaxGroup];
     // MIXED: the texel frame in FP64 (scattering.h:134-136 clamp, frame of
@@ -1549,14 +1618,11 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
     float3 acc[kDensMaxGroup];
 #pragma unroll
     for (int j = 0; j < kDensMaxGroup; ++j) acc[j] = make_float3(0.f, 0.f, 0.f);
-    // (sum, compensation) x 3 x G per thread, element e at accs[e * kDensThreads]:
-    // consecutive threads use consecutive banks, offsets are immediates
-    volatile float* accs = S.acc + tid;
     if (MX) {
 #pragma unroll
       for (int e = 0; e < 6 * kDensMaxGroup; ++e) accs[e * kDensThreads] = 0.f;
     }
-    for (int l = 0; l < NT; ++l) {
+    for (int l = ls * nq; l < l_end; ++l) {
       const DensTheta t = S.th[l];
       if (TWO) {
         const float4* Pl = S.P2 + (size_t)(cl * NT + l) * 3 * SL;
@@ -1593,7 +1659,7 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
             dens_row<false, CL, 0>(S, t, l, NT, Pl, q, sx, sy, G, pc, acc);
         }
       }
-      if (MX && ((l + 1) % kDensKahanRows == 0 || l == NT - 1)) {
+      if (MX && ((l + 1) % kDensKahanRows == 0 || l == l_end - 1)) {
         // Kahan sum over theta rows of the FP32 sums over kDensKahanRows rows
 #pragma unroll
         for (int j = 0; j < kDensMaxGroup; ++j) {
@@ -1608,19 +1674,34 @@ __device__ void tile_density(const DevAtmo& a, int order, int tile, unsigned cha
     }
 #pragma unroll
     for (int j = 0; j < kDensMaxGroup; ++j) {
-      if (j < G && grp * G + j < NNU) {
-        const int x = (grp * G + j) * a.sc_mus + si;
-        float* row = a.dens + ((size_t)zi * a.sc_mu + y) * 3 * a.Wd;
+      if (sh.LS > 1) {
+        if (!MX) {
+          accs[(3 * j) * kDensThreads] = acc[j].x;
+          accs[(3 * j + 1) * kDensThreads] = acc[j].y;
+          accs[(3 * j + 2) * kDensThreads] = acc[j].z;
+        }
+      } else if (j < G && grp * G + j < NNU) {
         float3 o = acc[j];
         if (MX)
           o = make_float3(accs[(6 * j) * kDensThreads] - accs[(6 * j + 3) * kDensThreads],
                           accs[(6 * j + 1) * kDensThreads] - accs[(6 * j + 4) * kDensThreads],
                           accs[(6 * j + 2) * kDensThreads] - accs[(6 * j + 5) * kDensThreads]);
-        // order 2: an end's sum holds one direction of each mirror pair
-        if (TWO && ((j == 0 && lo1) || (j == jh && hi1))) o = o * 2.0f;
-        row[x] = store_round(o.x, a.f16);
-        row[a.Wd + x] = store_round(o.y, a.f16);
-        row[2 * a.Wd + x] = store_round(o.z, a.f16);
+        store(j, o);
+      }
+    }
+  }
+  if (sh.LS > 1) {
+    // the shares of the theta rows, from the threads of the same texel
+    __syncthreads();
+    if (active && ls == 0) {
+      for (int j = 0; j < G && grp * G + j < NNU; ++j) {
+        float3 o = make_float3(0.f, 0.f, 0.f);
+        for (int h = 0; h < sh.LS; ++h) {
+          volatile float* p = accs + h * cap + (MX ? 6 : 3) * j * kDensThreads;
+          o = o + make_float3(p[0], p[kDensThreads], p[2 * kDensThreads]);
+          if (MX) o = o + make_float3(p[3 * kDensThreads], p[4 * kDensThreads], p[5 * kDensThreads]) * -1.0f;
+        }
+        store(j, o);
       }
     }
   }
@@ -2019,15 +2100,29 @@ constexpr int kMsSlabs = 4;
 constexpr int kMsWideThreads = 1024;
 constexpr int kMsRowBytes = 96 * 1024;  // shared memory for the rows of a tile (records + slabs)
 struct MSShape {
-  int R;         // rows per tile
+  int R;         // rows per tile, times SG
+  int SG;        // sample groups: each of a row's SG groups is a row of the tile with a share of the samples
+  int NS;        // samples of a group
   int TPT;       // texels per thread
   int slab_row;  // floats per slab plane: W, a zero guard slice and one zero entry, rounded up to 4
 };
-__host__ __device__ inline MSShape ms_shape(int W, int sc_mus, int steps, int threads) {
+// Tables of fewer tiles than the GPU has SMs split the samples of a row among up
+// to kMsMaxSplit rows of the tile, whose sums meet at the end: what bounds them is
+// the latency of a tile's samples, one after the other (smoke sizes, 16 tiles:
+// 26.6 -> 12.3 us). More tiles than that gain nothing and pay each tile's set-up
+// again (dump sizes, 256 tiles: 28.7 us split or not; a batch of 20 of them 0.277
+// -> 0.385 ms).
+constexpr int kMsMaxSplit = 8;
+__host__ __device__ inline MSShape ms_shape(int W, int sc_mus, int steps, int rows, int threads) {
   MSShape m;
   m.slab_row = (W + sc_mus + 1 + 3) & ~3;
-  const int row_bytes = (int)sizeof(MSRec) * (steps + 1) + kMsSlabs * 3 * (int)sizeof(float) * m.slab_row;
+  m.NS = steps + 1;
+  const int row_bytes = (int)sizeof(MSRec) * m.NS + kMsSlabs * 3 * (int)sizeof(float) * m.slab_row;
   m.R = W <= threads ? min(threads / W, max(1, kMsRowBytes / row_bytes)) : 1;
+  m.SG = 1;
+  while (m.SG < kMsMaxSplit && 2 * m.SG <= m.R && rows * m.SG < kFillTiles * m.R) m.SG *= 2;
+  m.R -= m.R % m.SG;
+  m.NS = (m.NS + m.SG - 1) / m.SG;
   m.TPT = (m.R * W + threads - 1) / threads;
   return m;
 }
@@ -2055,12 +2150,12 @@ __host__ __device__ inline int ms_variant(int W, int sc_mus) {
   return W <= kThreads ? 0 : (W <= kMsMidThreads ? kMsMid : kMsWide);
 }
 __host__ __device__ inline int tiles_multiple(int W, int sc_mus, int steps, int sc_mu, int sc_r, int threads) {
-  const MSShape m = ms_shape(W, sc_mus, steps, threads);
-  return (sc_mu * sc_r + m.R - 1) / m.R;
+  const MSShape m = ms_shape(W, sc_mus, steps, sc_mu * sc_r, threads);
+  return (sc_mu * sc_r * m.SG + m.R - 1) / m.R;
 }
-__host__ __device__ inline size_t ms_smem(int W, int steps, int sc_mus, int threads) {
-  const MSShape m = ms_shape(W, sc_mus, steps, threads);
-  return align16(sizeof(MSRec) * (size_t)m.R * (steps + 1)) + kMsSlabs * 3 * sizeof(float) * (size_t)m.R * m.slab_row;
+__host__ __device__ inline size_t ms_smem(int W, int steps, int sc_mus, int rows, int threads) {
+  const MSShape m = ms_shape(W, sc_mus, steps, rows, threads);
+  return align16(sizeof(MSRec) * (size_t)m.R * m.NS) + kMsSlabs * 3 * sizeof(float) * (size_t)m.R * m.slab_row;
 }
 
 // Position t in [0, n - 1] within a row of n texels as (i0, f): texel i0 in
@@ -2091,10 +2186,12 @@ template <bool MX, int TPT, int NMC, int WC, int NTH>
 __device__ void tile_multiple(const DevAtmo& a, int order, int tile, unsigned char* smem) {
   const int W = WC ? WC : a.W, nrows = a.sc_mu * a.sc_r, NM = NMC ? NMC : a.sc_mus;
   const int nth = NTH;
-  const MSShape sh = ms_shape(W, NM, a.ms_steps, nth);
-  const int row0 = tile * sh.R;
-  const int nrow = min(sh.R, nrows - row0);
-  const int N = a.ms_steps, NS = N + 1;
+  const MSShape sh = ms_shape(W, NM, a.ms_steps, nrows, nth);
+  // a row of the tile, lr, is group lr % SG of the samples of table row row0 + lr / SG
+  const int SG = WC && WC == NTH ? 1 : sh.SG;
+  const int row0 = tile * (sh.R / SG);
+  const int nrow = min(sh.R / SG, nrows - row0) * SG;
+  const int NS = sh.NS, N = NS - 1;  // samples of a group
   const int tid = threadIdx.x;
   constexpr int SRC = NMC ? (WC + NMC + 1 + 3) & ~3 : 0;
   const int SR = SRC ? SRC : sh.slab_row;          // slab plane stride
@@ -2113,18 +2210,24 @@ __device__ void tile_multiple(const DevAtmo& a, int order, int tile, unsigned ch
   {  // this tile's sample records, their density row offsets bounded to the table
     static_assert(sizeof(MSRec) == 4 * sizeof(int4) && offsetof(MSRec, off) == 3 * sizeof(int4),
                   "MSRec: four 16-byte words, the offsets last");
-    const int4* src = reinterpret_cast<const int4*>(a.g_ms + (size_t)row0 * NS);
     int4* dst = reinterpret_cast<int4*>(rec);
     const int omax = (a.sc_r * a.sc_mu - 1) * (3 * a.Wd / 4);  // start of the table's last row
     for (int k = tid; k < nrow * NS; k += nth) {
-      int4 o = __ldg(src + 4 * k + 3);
+      const int lr = k / NS, i = (lr % SG) * NS + (k - lr * NS);
+      const int4* src = reinterpret_cast<const int4*>(a.g_ms + (size_t)(row0 + lr / SG) * (a.ms_steps + 1) + min(i, a.ms_steps));
+      int4 o = __ldg(src + 3);
       o.x = min(max(o.x, 0), omax);
       o.y = min(max(o.y, 0), omax);
       o.z = min(max(o.z, 0), omax);
       o.w = min(max(o.w, 0), omax);
-      dst[4 * k] = __ldg(src + 4 * k);
-      dst[4 * k + 1] = __ldg(src + 4 * k + 1);
-      dst[4 * k + 2] = __ldg(src + 4 * k + 2);
+      int4 d = __ldg(src), t = __ldg(src + 1);
+      if (i > a.ms_steps) {  // past the row's samples: a sample of weight 0
+        d.z = d.w = 0;
+        t.x = 0;
+      }
+      dst[4 * k] = d;
+      dst[4 * k + 1] = t;
+      dst[4 * k + 2] = __ldg(src + 2);
       dst[4 * k + 3] = o;
     }
   }
@@ -2203,7 +2306,7 @@ __device__ void tile_multiple(const DevAtmo& a, int order, int tile, unsigned ch
     c_e[j] = c_lr[j] * 3 * SR;
     c_ro[j] = c_lr[j] * NS;
     const int slice = c_x[j] / NM;
-    const RowGeo& rg = a.g_rows[row0 + c_lr[j]];
+    const RowGeo& rg = a.g_rows[row0 + c_lr[j] / SG];
     const ColGeo& cg = a.g_cols[c_x[j]];
     float mu_s, nu, rmus;
     texel_mus_nu<MX>(rg, cg, mu_s, nu, rmus);
@@ -2418,26 +2521,33 @@ __device__ void tile_multiple(const DevAtmo& a, int order, int tile, unsigned ch
     cur ^= pair;
     nxt ^= pair;
   }
-  // the ends' results to the texels that the clamp moves to them (the loops
-  // end with a barrier: the slabs are no longer read)
+  // the groups' sums of each texel, and the ends' results to the texels that the
+  // clamp moves to them (the loops end with a barrier: the slabs are no longer read)
+  const int n_keep = SG > 1 ? nx_tex : n_end;
 #pragma unroll
   for (int j = 0; j < TPT; ++j) {
     const int k = tid + j * nth;
     part[j] = make_float3(acc[j].s.x - acc[j].c.x, acc[j].s.y - acc[j].c.y, acc[j].s.z - acc[j].c.z);
-    if (k < n_end) {
+    if (k < n_keep) {
       slab[k] = part[j].x;
-      slab[n_end + k] = part[j].y;
-      slab[2 * n_end + k] = part[j].z;
+      slab[n_keep + k] = part[j].y;
+      slab[2 * n_keep + k] = part[j].z;
     }
   }
   __syncthreads();
   // outputs: delta multiple scattering and the final table (:91-92)
 #pragma unroll
   for (int j = 0; j < TPT; ++j) {
-    if (has_tex[j]) {
-      const size_t t = (size_t)(row0 + c_lr[j]) * W + c_x[j];
+    if (has_tex[j] && c_lr[j] % SG == 0) {
+      const size_t t = (size_t)(row0 + c_lr[j] / SG) * W + c_x[j];
       float3 ms = part[j];
-      if (c_from[j] >= 0) ms = make_float3(slab[c_from[j]], slab[n_end + c_from[j]], slab[2 * n_end + c_from[j]]);
+      const int k = tid + j * nth, from = c_from[j] >= 0 ? c_from[j] : k;
+      if (SG > 1 || from != k) {
+        const int stride = from < n_end ? 2 * NM : W - 2 * NM;
+        ms = make_float3(0.f, 0.f, 0.f);
+        for (int g = 0; g < SG; ++g)
+          ms = ms + make_float3(slab[from + g * stride], slab[n_keep + from + g * stride], slab[2 * n_keep + from + g * stride]);
+      }
       a.dms[t] = store_round4(make_float4(ms.x, ms.y, ms.z, 0.f), a.f16);
       const float pr = phase_rayleigh(c_nu[j]);
       if (!MX) {
@@ -2491,22 +2601,23 @@ __host__ __device__ inline int tiles_transmittance(int tr_mu, int tr_r) {
   return (tr_mu * tr_r + kTrTexels - 1) / kTrTexels;
 }
 __host__ __device__ inline int tiles_rows(int W, int sc_mu, int sc_r) {
-  const int R = rows_per_tile(W);
+  const int R = ss_shape(W, sc_mu * sc_r).R;
   return (sc_mu * sc_r + R - 1) / R;
 }
 __host__ __device__ inline int tiles_direct(int ir_mus, int ir_r) { return (ir_mus * ir_r + kThreads - 1) / kThreads; }
 __host__ __device__ inline int tiles_density(const DevAtmo& a) {
   return dens_shape(a.sc_r, a.sc_mu, a.sc_mus, a.sc_nu, a.dens_S, a.dens_chunk).tiles;
 }
-__host__ __device__ inline size_t ss_smem(int W, int steps, int sc_mus, int sc_nu) {
-  (void)sc_mus;
-  (void)sc_nu;
-  const int R = rows_per_tile(W);
-  return align16(sizeof(RowGeo) * R) + sizeof(SSRec) * (size_t)R * (steps + 1);
+__host__ __device__ inline size_t ss_smem(int W, int steps, int rows) {
+  // (of the unsplit tile: what a launch may ask for does not depend on the split)
+  const SSShape s = ss_shape(W, rows);
+  const int R = s.R * s.SG;
+  const size_t rec = sizeof(SSRec) * (size_t)R * (steps + 1), sums = s.SG > 1 ? 6 * sizeof(float) * kThreads : 0;
+  return align16(sizeof(RowGeo) * R) + (rec > sums ? rec : sums);
 }
 __host__ __device__ inline size_t density_smem(const DevAtmo& a, bool two, bool mixed, bool cl) {
   const DensShape d = dens_shape(a.sc_r, a.sc_mu, a.sc_mus, a.sc_nu, a.dens_S, a.dens_chunk);
-  return dens_layout(nullptr, a.dens_n, a.sc_nu, a.ir_mus, d.S, d.chunk, two, mixed, cl, nullptr);
+  return dens_layout(nullptr, a.dens_n, a.sc_nu, a.ir_mus, d.S, d.chunk, two, mixed, cl, d.LS, nullptr);
 }
 // Density variants: the occupancy variant (0..2), plus kDensClamped for the
 // clamped interval tables.
