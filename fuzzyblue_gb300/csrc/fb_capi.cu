@@ -578,16 +578,16 @@ void plan_group(Plan& P, const std::vector<DevAtmo>& A, const std::vector<int>& 
       t1.push_back(fb::tiles_direct(a.ir_mus, a.ir_r));
       if (a.order >= 2) {
         multi.push_back(j);
-        t2.push_back(fb::tiles_msrec(a.sc_mu, a.sc_r, a.ms_steps));
+        t2.push_back(fb::ms_fused(a.ss_steps, a.ms_steps) ? 0 : fb::tiles_msrec(a.sc_mu, a.sc_r, a.ms_steps));
         t3.push_back(fb::tiles_densgeo(a.sc_r, a.dens_n));
       }
       L.smem = std::max(L.smem, fb::ss_smem(a.W, a.ss_steps, a.sc_mu * a.sc_r));
       L.texels += (uint64_t)a.W * a.sc_mu * a.sc_r + (uint64_t)a.ir_mus * a.ir_r;
     }
-    add_segment(P, L, 0, group, t0);
-    add_segment(P, L, 1, group, t1);
-    add_segment(P, L, 2, multi, t2);
-    add_segment(P, L, 3, multi, t3);
+    add_segment(P, L, 0, multi, t3);
+    add_segment(P, L, 1, group, t0);
+    add_segment(P, L, 2, group, t1);
+    add_segment(P, L, 3, multi, t2);
     L.nseg = 4;
     P.launches.push_back(L);
   }

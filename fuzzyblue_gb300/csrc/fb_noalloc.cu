@@ -241,8 +241,9 @@ extern "C" int fb_atmosphere_build_noalloc(void* stream, const fb_params* p, voi
            0, 1, fb::kThreads, 0);
   if (!rc)
     rc = add(fb::kPassSingle, 0,
-             {fb::tiles_rows(d.W, d.sc_mu, d.sc_r), fb::tiles_direct(d.ir_mus, d.ir_r),
-              multi ? fb::tiles_msrec(d.sc_mu, d.sc_r, d.ms_steps) : 0, multi ? fb::tiles_densgeo(d.sc_r, d.dens_n) : 0},
+             {multi ? fb::tiles_densgeo(d.sc_r, d.dens_n) : 0, fb::tiles_rows(d.W, d.sc_mu, d.sc_r),
+              fb::tiles_direct(d.ir_mus, d.ir_r),
+              multi && !fb::ms_fused(d.ss_steps, d.ms_steps) ? fb::tiles_msrec(d.sc_mu, d.sc_r, d.ms_steps) : 0},
              fb::ss_smem(d.W, d.ss_steps, d.sc_mu * d.sc_r), 1, fb::kThreads, 0);
   const int ms_variant = fb::ms_variant(d.W, d.sc_mus), ms_block = fb::ms_layout(ms_variant).threads;
   const int ms_tpt = fb::ms_shape(d.W, d.sc_mus, d.ms_steps, d.sc_mu * d.sc_r, ms_block).TPT;

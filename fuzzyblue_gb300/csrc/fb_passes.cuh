@@ -5,11 +5,12 @@
 // Launch structure (one launch per pass group, any number of atmospheres):
 //   k_transmittance  transmittance.comp                      warp per texel, two per work item
 //                    geometry tables: rows, x columns (seg 0) thread per entry
-//   k_single         single_scattering.comp  (segment 0)     CTA per (mu, r) row(s), texels
+//   k_single         density r / theta records (segment 0)   thread per record
+//                    single_scattering.comp  (segment 1)     CTA per (mu, r) row(s), texels
 //                                                            to threads nu slice fastest
-//                    direct_irradiance.comp  (segment 1)     thread per texel
-//                    multiple-scattering samples (seg 2)     thread per (row, sample)
-//                    density r / theta records (segment 3)   thread per record
+//                    direct_irradiance.comp  (segment 2)     thread per texel
+//                    multiple-scattering samples (seg 3)     thread per (row, sample), where
+//                                                            the rows' tiles do not write them
 //   k_density        scattering_density.comp (segment 0)     CTA per (r, mu_s, mu-chunk)
 //   k_density_arcs     the same for orders >= 3              CTA per (r, mu_s columns, 32 mu rows)
 //                    indirect_irradiance.comp (segment 1)    CTA per irradiance r row (up to 64 texels);
@@ -501,21 +502,22 @@ __host__ __device__ inline SSShape ss_shape(int W, int rows) {
 
 // ======================================================= MS sample records ===
 // multiple_scattering.comp:19-40, the parts that depend on the view ray and
-// the sample only (single-scattering launch, segment 2): the sample distance
-// and radius, the transmittance from the texel times dx and the trapezoid
-// weight, and the four density rows around the sample's (mu, r) with their
-// bilinear weights.
-template <bool MX> __device__ void tile_msrec(const DevAtmo& a, int tile) {
-  const int NS = a.ms_steps + 1;
-  const int k = tile * kThreads + threadIdx.x;
-  const int nrows = a.sc_mu * a.sc_r;
-  if (k >= nrows * NS) return;
-  const int row = k / NS, i = k % NS, N = a.ms_steps;
-  const RowGeo ri = a.g_rows[row];
+// the sample only: the sample distance and radius, the transmittance from the
+// texel (tv) times dx and the trapezoid weight, and the four density rows
+// around the sample's (mu, r) with their bilinear weights. Where single and
+// multiple scattering have the same number of steps, the single-scattering tile
+// of the row writes them with its own records, which need the same tv; else they
+// are items of their own (single-scattering launch, segment 3). Those items are
+// bound by FP64 at the launch's end: writing them along took the launch of 20
+// half-class atmospheres from 0.455 to 0.394 ms (with the theta records first and
+// spread over SMs), of 16 default ones from 4.56 to 4.46.
+__host__ __device__ inline bool ms_fused(int ss_steps, int ms_steps) { return ss_steps == ms_steps; }
+template <bool MX>
+__device__ __forceinline__ void ms_record(const DevAtmo& a, const RowGeo& ri, int row, int i, float3 tv) {
+  const int N = a.ms_steps, NS = N + 1;
   MSRec o;
   o.pad0 = o.pad1 = o.pad2 = 0.f;
   const float w = (i == 0 || i == N) ? 0.5f : 1.0f;
-  float3 tv;
   Axis ay, az;
   float dx;
   if (!MX) {
@@ -525,7 +527,6 @@ template <bool MX> __device__ void tile_msrec(const DevAtmo& a, int tile) {
     const float d = float(i) * dx;
     const float r_i = G.clamp_radius(sqrtf(d * d + ri.two_r_mu * d + ri.rr));
     const float mu_i = clamp_cosine((ri.r_mu + d) / r_i);
-    tv = G.tr_segment(a, ri.r, ri.mu, d, ri.ground);
     az = make_axis(G.u_r(a, r_i), a.sc_r);
     ay = make_axis(G.u_mu(a, r_i, mu_i, ri.ground), a.sc_mu);
     o.d = d;
@@ -540,7 +541,6 @@ template <bool MX> __device__ void tile_msrec(const DevAtmo& a, int tile) {
     q = fmin(fmax(q, 0.0), G.H2);
     const float r_i = sqrtf((float)q + G.R * G.R);
     sd = fmin(fmax(sd, -(double)r_i), (double)r_i);
-    tv = G.tr_segment(a, ri.q, ri.s, d, ri.ground);
     az = axis_texel(G.sc_r_texel(q), a.sc_r);
     ay = axis_texel(G.sc_mu_texel(q, sd, ri.ground), a.sc_mu);
     o.d = (float)d;
@@ -559,7 +559,26 @@ template <bool MX> __device__ void tile_msrec(const DevAtmo& a, int tile) {
   o.off[1] = (az.i0 * a.sc_mu + ay.i1) * rs;
   o.off[2] = (az.i1 * a.sc_mu + ay.i0) * rs;
   o.off[3] = (az.i1 * a.sc_mu + ay.i1) * rs;
-  a.g_ms[k] = o;
+  a.g_ms[(size_t)row * NS + i] = o;
+}
+template <bool MX> __device__ void tile_msrec(const DevAtmo& a, int tile) {
+  const int NS = a.ms_steps + 1;
+  const int k = tile * kThreads + threadIdx.x;
+  const int nrows = a.sc_mu * a.sc_r;
+  if (k >= nrows * NS) return;
+  const int row = k / NS, i = k % NS, N = a.ms_steps;
+  const RowGeo ri = a.g_rows[row];
+  float3 tv;
+  if (!MX) {
+    Geo32 G;
+    G.init(a);
+    tv = G.tr_segment(a, ri.r, ri.mu, float(i) * (ri.dist / float(N)), ri.ground);
+  } else {
+    GeoMx G;
+    G.init(a);
+    tv = G.tr_segment(a, ri.q, ri.s, double(i) * (ri.distd / double(N)), ri.ground);
+  }
+  ms_record<MX>(a, ri, row, i, tv);
 }
 
 __host__ __device__ inline int tiles_msrec(int sc_mu, int sc_r, int ms_steps) {
@@ -568,14 +587,14 @@ __host__ __device__ inline int tiles_msrec(int sc_mu, int sc_r, int ms_steps) {
 
 // =================================================== density r / theta ===
 // scattering_density.comp:36-60, the parts that depend on r and the theta
-// row only (single-scattering launch, segment 3): per r slice the r axis of
+// row only (single-scattering launch, segment 0): per r slice the r axis of
 // the 3D tables; per (r slice, theta row) the direction's cosine, the solid
 // angle of its row, the ground hit (distance, transmittance x albedo / pi)
 // and the mu axis of the lookup.
 template <bool MX> __device__ void tile_densgeo(const DevAtmo& a, int tile) {
   const int NT = a.dens_n;
-  const int k = tile * kThreads + threadIdx.x;
-  if (k >= a.sc_r * (NT + 1)) return;
+  const int k = tile * kGeoEntries + threadIdx.x;  // FP64-bound, spread over SMs as tile_geometry
+  if (threadIdx.x >= kGeoEntries || k >= a.sc_r * (NT + 1)) return;
   if (k < a.sc_r) {
     DensZ o;
     o.pad = 0;
@@ -661,7 +680,7 @@ template <bool MX> __device__ void tile_densgeo(const DevAtmo& a, int tile) {
 }
 
 __host__ __device__ inline int tiles_densgeo(int sc_r, int dens_n) {
-  return (sc_r * (dens_n + 1) + kThreads - 1) / kThreads;
+  return (sc_r * (dens_n + 1) + kGeoEntries - 1) / kGeoEntries;
 }
 
 // ============================================================ S: single ===
@@ -692,6 +711,7 @@ __device__ void tile_single(const DevAtmo& a, int tile, unsigned char* smem) {
   const int tid = threadIdx.x;
   if (tid < nrow) rows[tid] = a.g_rows[row0 + tid];
   __syncthreads();
+  const bool records = a.order >= 2 && ms_fused(a.ss_steps, a.ms_steps);
   // Per (row, sample): the view ray point, the transmittance to it, the
   // densities there and the parts of the sun lookup that depend on it only.
   for (int k = tid; k < nrow * NS; k += kThreads) {
@@ -762,6 +782,7 @@ __device__ void tile_single(const DevAtmo& a, int tile, unsigned char* smem) {
       o.y1 = ay.i1;
       o.fy = ay.f;
     }
+    if (records) ms_record<MX>(a, ri, row0 + k / NS, i, tv);
     const float wr = w * rho_r, wm = w * rho_m;
     o.trx = tv.x * wr;
     o.try_ = tv.y * wr;
@@ -873,14 +894,12 @@ template <bool MX> __global__ void __launch_bounds__(kThreads, 4) k_single(Launc
   int seg, job, tile;
   int taken = 0;
   while (next_item(L, seg, job, tile, taken)) {
-    if (seg == 0) {
-      const DevAtmo& a = L.atm[job];
-      if (ss_shape(a.W, a.sc_mu * a.sc_r).SG > 1) tile_single<MX, true>(a, tile, smem);
-      else tile_single<MX, false>(a, tile, smem);
-    }
-    else if (seg == 1) tile_direct<MX>(L.atm[job], tile);
-    else if (seg == 2) tile_msrec<MX>(L.atm[job], tile);
-    else tile_densgeo<MX>(L.atm[job], tile);
+    const DevAtmo& a = L.atm[job];
+    if (seg == 0) tile_densgeo<MX>(a, tile);  // first: the longest items in FP64
+    else if (seg == 1 && ss_shape(a.W, a.sc_mu * a.sc_r).SG > 1) tile_single<MX, true>(a, tile, smem);
+    else if (seg == 1) tile_single<MX, false>(a, tile, smem);
+    else if (seg == 2) tile_direct<MX>(a, tile);
+    else tile_msrec<MX>(a, tile);
   }
 }
 
