@@ -602,18 +602,19 @@ void plan_group(Plan& P, const std::vector<DevAtmo>& A, const std::vector<int>& 
     if (!arcs.empty()) {
       PlannedLaunch D = mk(fb::kPassDensity, n);
       std::vector<int> t0, t1;
-      int gi = 0;
+      int gi = 0, tiles = 0;
       for (int j : arcs) {
         const DevAtmo& a = A[j];
         const fb::ArcShape sh = fb::arc_shape(a.sc_r, a.sc_mu, a.sc_mus, a.sc_nu);
         gi = std::max(gi, sh.gi);
         t0.push_back(sh.tiles);
+        tiles += sh.tiles;
         t1.push_back(fb::tiles_indirect(a.ir_mus, a.ir_r, a.irr_n, a.sc_nu, false));
         D.texels += (uint64_t)a.W * a.sc_mu * a.sc_r + (uint64_t)a.ir_mus * a.ir_r;
       }
       D.block = fb::kArcThreads;
       D.variant = fb::arc_variant(gi);
-      D.arc_rows = fb::arc_launch_rows(arcs, [&](int j) -> const DevAtmo& { return A[j]; }, fb::arc_ctas(gi), &D.smem);
+      D.arc_rows = fb::arc_launch_rows(arcs, [&](int j) -> const DevAtmo& { return A[j]; }, tiles, fb::arc_ctas(gi), &D.smem);
       for (int j : arcs)
         D.smem = std::max(D.smem, fb::indirect_smem(A[j].irr_n, A[j].sc_nu, A[j].W, false, D.block));
       add_segment(P, D, 0, arcs, t0);

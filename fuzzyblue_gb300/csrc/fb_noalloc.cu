@@ -251,7 +251,7 @@ extern "C" int fb_atmosphere_build_noalloc(void* stream, const fb_params* p, voi
     if (n >= 3 && d.arcs) {
       const fb::ArcShape sh = fb::arc_shape(d.sc_r, d.sc_mu, d.sc_mus, d.sc_nu);
       size_t sm = 0;
-      arc_rows = fb::arc_launch_rows(std::vector<int>{0}, [&](int) -> const fb::DevAtmo& { return d; }, fb::arc_ctas(sh.gi), &sm);
+      arc_rows = fb::arc_launch_rows(std::vector<int>{0}, [&](int) -> const fb::DevAtmo& { return d; }, sh.tiles, fb::arc_ctas(sh.gi), &sm);
       sm = std::max(sm, fb::indirect_smem(d.irr_n, d.sc_nu, d.W, false, fb::kArcThreads));
       rc = add(fb::kPassDensity, n, {sh.tiles, fb::tiles_indirect(d.ir_mus, d.ir_r, d.irr_n, d.sc_nu, false)}, sm, 1,
                fb::kArcThreads, fb::arc_variant(sh.gi));
