@@ -19,9 +19,10 @@
 // directions. Measured against the direct sums (tile_density), density of order
 // 3 with its indirect irradiance: 16 default atmospheres 6.46 -> 1.98 ms, one of
 // twice the size in every dimension (16 nu slices) 6.58 -> 3.79 ms, one default
-// atmosphere 0.461 -> 0.156 ms, with the same errors against FP64. Bound by the shared-memory pipe (76 %
-// of its wavefronts; six 8-byte loads per texel and knot) and, between the
-// batches of theta rows, by the latency of building the next ones.
+// atmosphere 0.461 -> 0.156 ms, with the same errors against FP64. Bound by the
+// shared-memory pipe (76 % of its wavefronts; six 8-byte loads per texel and
+// knot) and, between the batches of theta rows, by the latency of building the
+// next ones.
 //
 // The weights are c_m = A t1_m + B t1_m rs3_m per channel (PhaseCoef) with A
 // and B constant in the tile: the running sums are kept for t1 and t1 rs3 and

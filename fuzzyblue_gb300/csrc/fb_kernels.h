@@ -9,11 +9,11 @@ namespace fb {
 enum PassKind { kPassTransmittance = 0, kPassSingle = 1, kPassDensity = 2, kPassMultiple = 3 };
 
 // Kernel of (mode, pass, texels-per-thread, variant, order 2). Multiple
-// scattering: variant 0 / 1 = CTAs of kThreads with registers for 4 / 3 CTAs
-// per SM (tpt 1), variant 2 / 3 = CTAs of kMsWideThreads / kMsMidThreads
-// (tpt 1 or 2). Density:
-// variant 0 / 1 = registers for 4 / 3 CTAs per SM; order2 selects the launch
-// of order 2 (it reads the single-scattering tables).
+// scattering: the variants of ms_variant (by the row's layout; 0 / 1 and 4 / 5
+// = registers for 4 / 3 CTAs per SM). Density: occupancy variant 0-2, +
+// kDensClamped with exact-size interval tables; order2 selects the launch of
+// order 2 (it reads the single-scattering tables); from kDensArcs, orders >= 3
+// by arcs, by the nu texels of a thread.
 const void* kernel_plain(int pass, int tpt, int variant, bool order2);
 const void* kernel_mixed(int pass, int tpt, int variant, bool order2);
 

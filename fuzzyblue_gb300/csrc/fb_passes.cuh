@@ -392,7 +392,6 @@ template <bool MX> __device__ void tile_geometry(const DevAtmo& a, int tile) {
     const int row = k - a.W;
     const uint32_t y = (uint32_t)(row % a.sc_mu), z = (uint32_t)(row / a.sc_mu);
     RowGeo o;
-    o.mu_lo = o.om_hi = o.om_lo = 0.f;
     if (!MX) {
       Geo32 G;
       G.init(a);
@@ -424,7 +423,6 @@ template <bool MX> __device__ void tile_geometry(const DevAtmo& a, int tile) {
       o.mu_lo = (float)(p.mu - (double)o.mu);
       o.om_hi = (float)o.one_m_mu2;
       o.om_lo = (float)(o.one_m_mu2 - (double)o.om_hi);
-      o.rr = o.two_r_mu = o.r_mu = 0.f;
     }
     a.g_rows[row] = o;
   } else if (MX) {

@@ -5,9 +5,11 @@
 // candidate: every valid scattering-density tile shape (mu_s columns x mu
 // rows per 128-thread block) in the three occupancy variants of the density
 // kernel (4, 3 or 5 resident blocks per SM), each with power-of-two and with
-// exact-size interval tables, then both variants of the multiple-scattering
-// kernel. The fastest of each is
-// kept in the builder's tuning table, which every later build consults.
+// exact-size interval tables, timed on the order-2 launch where the later
+// orders go by arcs (which have a shape of their own) and on order 3
+// otherwise; then both variants of the multiple-scattering kernel. The fastest
+// of each is kept in the builder's tuning table, which every later build
+// consults.
 #include <cuda_runtime.h>
 
 #include <algorithm>
