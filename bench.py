@@ -146,15 +146,15 @@ def max_over_ranks(world, v):
 
 
 # ------------------------------------------------------------- roofline ---
-# The roofline of the dominant launch (scattering density of order n >= 3 plus
-# the indirect irradiance of order n - 1) is reported on the FP32 pipe: the
+# The roofline of the longest launch (scattering density of order 2 plus the
+# indirect irradiance of order 1) is reported on the FP32 pipe: the
 # FLOPs the kernel executes per direction evaluation (measured with ncu on the
 # same launch, a committed profile summary) times the directions of the
 # launch, over its CUDA-event time. Beside it: the reference's quadrature
 # arithmetic per output texel, op-counted on the oracle's restatement over the
 # first 16 atmospheres of this workload (`python oracle/count_flops.py`; adds,
 # muls, divs, sqrts and transcendentals one FLOP each, sampler filtering and
-# literal-only expressions not counted; 162.6 FLOPs per direction at n >= 3).
+# literal-only expressions not counted; 261 FLOPs per direction at order 2).
 FLOP_PER_TEXEL = {
     "transmittance": 28311.7,
     "direct_irradiance": 34.0,
@@ -166,21 +166,22 @@ FLOP_PER_TEXEL = {
     "multiple_scattering": 8332.2,
 }
 FLOP_PER_ATMOSPHERE = 350185724984.0  # default sizes, 4 orders (same count)
-# Counts of the dominant launch measured with ncu on the kernel sources whose
+# Counts of the longest launch measured with ncu on the kernel sources whose
 # SHA-256 (first 16 hex digits, over KERNEL_SOURCES) is `sources`: the
 # executed FP32 FLOPs and thread instructions per direction evaluation (a
 # --set full capture of 16 atmospheres) and the DRAM bytes per launch (the same
 # capture, scaled to the launch's atmospheres). The commands are in the profile
 # summaries named by `profile`. When the sources on disk differ, the roofline
 # is reported with "stale": true.
-KERNEL_SOURCES = ("fuzzyblue_gb300/csrc/fb_passes.cuh", "fuzzyblue_gb300/csrc/fb_device.cuh")
+KERNEL_SOURCES = ("fuzzyblue_gb300/csrc/fb_passes.cuh", "fuzzyblue_gb300/csrc/fb_device.cuh",
+                  "fuzzyblue_gb300/csrc/fb_density_arcs.cuh")
 DENSITY_NCU = {
-    "sources": "3c8e1ac1b66b0be0",
+    "sources": "5c343f3e91350296",
     "profile": "profiles/passes_uniform16_mixed_ncu.md",
     "atmospheres": 16,
-    "fp32_flop_per_direction_order3": 24.49,
-    "thread_instr_per_direction_order3": 20.54,
-    "dram_bytes_per_atmosphere_order3": 13.16e6,
+    "fp32_flop_per_direction_order2": 36.37,
+    "thread_instr_per_direction_order2": 26.88,
+    "dram_bytes_per_atmosphere_order2": 18.43e6,
 }
 
 
@@ -365,26 +366,26 @@ def run_ours(a):
         for r in launches:
             key = r["kernel"] + ("" if r["order"] == 0 else "_order%d" % min(r["order"], 3))
             kernels.setdefault(key, []).append(r)
-    dens = [r for launches in prof for r in launches if r["kernel"] == "density+indirect" and r["order"] >= 3]
+    dens = [r for launches in prof for r in launches if r["kernel"] == "density+indirect" and r["order"] == 2]
     dens_ms = sum(r["ms"] for r in dens) / max(len(dens), 1)
     sms = builder.sm_count
     # executed FP32 FLOPs per direction evaluation of this launch (ncu) and
     # the reference's quadrature FLOPs per texel (oracle op count)
     directions = a.batch * sizes[2] * 2 * params[0].density_samples ** 2
-    exec_per_dir = DENSITY_NCU["fp32_flop_per_direction_order3"]
+    exec_per_dir = DENSITY_NCU["fp32_flop_per_direction_order2"]
     stale = kernel_sources_sha() != DENSITY_NCU["sources"]
-    ref_flops = a.batch * (sizes[2] * FLOP_PER_TEXEL["density_order3"] + sizes[1] * FLOP_PER_TEXEL["indirect_order2"])
+    ref_flops = a.batch * (sizes[2] * FLOP_PER_TEXEL["density_order2"] + sizes[1] * FLOP_PER_TEXEL["indirect_order1"])
     mhz = (clk or {}).get("sm_mhz") or 2070.0
     peak = fp32_peak_tflops(sms, mhz)
     exec_flops = directions * exec_per_dir if exec_per_dir else None
     achieved = exec_flops / (dens_ms / 1e3) / 1e12 if exec_flops else None
     ref_achieved = ref_flops / (dens_ms / 1e3) / 1e12
-    traffic = DENSITY_NCU["dram_bytes_per_atmosphere_order3"] * a.batch
+    traffic = DENSITY_NCU["dram_bytes_per_atmosphere_order2"] * a.batch
     peaks = measured_peaks()
-    # the launch's binding limit is instruction issue: warp instructions per
+    # beside the shared-memory pipe the launch is bound by instruction issue: warp instructions per
     # launch (ncu's thread instructions per direction / 32) against one per
     # cycle per scheduler, 4 schedulers per SM
-    instr_per_dir = DENSITY_NCU["thread_instr_per_direction_order3"]
+    instr_per_dir = DENSITY_NCU["thread_instr_per_direction_order2"]
     issue = None
     if instr_per_dir:
         issue_achieved = directions * instr_per_dir / 32.0 / (dens_ms / 1e3) / 1e9
@@ -418,7 +419,7 @@ def run_ours(a):
                 "overlap": "each step built as %d batches of %d on two streams: a batch's copies overlap the next "
                            "batch's kernels" % (parts, sub)},
         "gpu_launches": sum(len(x) for x in prof),
-        "roofline": {"bound": "fp32", "kernel": "k_density (scattering density + indirect irradiance), order >= 3",
+        "roofline": {"bound": "fp32", "kernel": "k_density (scattering density + indirect irradiance), order 2",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak if achieved else None,
                      "peak_source": "152 SMs x 128 FP32 lanes x 2 FLOP x median SM clock under load (%d MHz); "
@@ -437,7 +438,7 @@ def run_ours(a):
                      "issue": issue,
                      "reference_algorithm": {
                          "achieved": ref_achieved, "frac": ref_achieved / peak,
-                         "flop_per_texel": FLOP_PER_TEXEL["density_order3"],
+                         "flop_per_texel": FLOP_PER_TEXEL["density_order2"],
                          "note": "the reference's quadrature arithmetic (oracle op count, oracle/count_flops.py) "
                                  "delivered per second: the kernel executes fewer FLOPs per direction than the "
                                  "reference's shader code (per-tile reduced tables replace the 4D lookups)"}},
