@@ -666,6 +666,21 @@ void plan_group(Plan& P, const std::vector<DevAtmo>& A, const std::vector<int>& 
   }
 }
 
+// Fewer mu_s columns per density tile where the tables of the default or tuned
+// shape, of exact size, would not fit in shared memory: many columns of few mu rows
+// with few nu slices (order 2 keeps at least 8 records per column), or beside the
+// longest ground rows. The shape changes no result.
+void limit_density_shape(DevAtmo& d, bool mixed) {
+  constexpr size_t limit = 226 * 1024;  // what a launch may use (227 KB, 1 KB of them static)
+  const fb::DensShape sh = fb::dens_shape(d.sc_r, d.sc_mu, d.sc_mus, d.sc_nu, d.dens_S, d.dens_chunk);
+  for (int S = sh.S; S > 1 && (fb::density_smem(d, true, mixed, true) > limit ||
+                               fb::density_smem(d, false, mixed, true) > limit);) {
+    S = (S + 1) / 2;
+    d.dens_S = S;
+    d.dens_chunk = sh.chunk;
+  }
+}
+
 void fill_devatmo(DevAtmo& d, const fb_params& p, const fbi::Tuning& tun) {
   std::memset(&d, 0, sizeof(d));
   const fb_params_raw& r = p.raw;
@@ -719,6 +734,7 @@ void fill_devatmo(DevAtmo& d, const fb_params& p, const fbi::Tuning& tun) {
   const fbi::TuneEntry* te = fbi::tuning_find(tun, d.sc_r, d.sc_mu, d.sc_mus, d.sc_nu, (int)p.precision);
   d.dens_S = te ? te->dens_S : 0;
   d.dens_chunk = te ? te->dens_chunk : 0;
+  limit_density_shape(d, p.precision == FB_PRECISION_MIXED);
   d.arc_ke = fb::arc_ground_knots(d.ir_mus, d.bottom, d.Hd);
   d.arcs = fb::arc_use(d);
 }

@@ -923,6 +923,9 @@ constexpr int kDensMaxGroup = 8;
 // tiles: one atmosphere of it would gain (117 -> 86 us), a batch of 20 lose (0.767
 // -> 0.841 ms), as every tile reads the tables of all theta rows.
 constexpr int kDensFillTiles = 100;
+// Nor those of more nu slices, whose tables leave no room for the sums of the
+// groups beside the longest ground rows (32 density samples, 4096 texels).
+constexpr int kDensSplitNu = 32;
 
 // Per-atmosphere tile shape of the density pass (host and device agree).
 struct DensShape {
@@ -943,7 +946,9 @@ __host__ __device__ inline DensShape dens_shape(int sc_r, int sc_mu, int sc_mus,
   const int per_col = sc_mu * d.NG;
   // (by the table's sizes alone: a tuned shape changes no sum)
   d.LS = 1;
-  while (d.LS < 4 && per_col * sc_mus * sc_r * d.LS < kDensFillTiles * kDensThreads && d.NG * 2 * d.LS <= kDensThreads) d.LS *= 2;
+  while (d.LS < 4 && per_col * sc_mus * sc_r * d.LS < kDensFillTiles * kDensThreads && d.NG * 2 * d.LS <= kDensThreads &&
+         sc_nu <= kDensSplitNu)
+    d.LS *= 2;
   const int threads = kDensThreads / d.LS;
   if (S_req > 0 && chunk_req > 0 && S_req * min(chunk_req, sc_mu) * d.NG <= threads) {
     d.S = min(S_req, sc_mus);
